@@ -17,6 +17,7 @@ ADAction recipes (reference file:line):
 """
 from __future__ import annotations
 
+import weakref
 from typing import Callable, List, Optional, Tuple
 
 import numpy as np
@@ -29,11 +30,17 @@ from .tensor import Tensor
 
 
 class GraphNode:
-    """The payload's place in the computation graph: parents + one ADAction per differentiable parent."""
+    """The payload's place in the computation graph: parents + one ADAction per differentiable parent. The payload owns
+    its node and not the other way round: a cycle between them would keep every result of a training step, and its device
+    memory, until the interpreter's cycle collector happened to run."""
 
     def __init__(self, payload: Tensor, parents: List[Tuple[Tensor, Callable[[Tensor], Tensor]]]):
-        self.payload = payload
+        self._payload = weakref.ref(payload)
         self.parents = parents  # (input tensor, error -> error for that input)
+
+    @property
+    def payload(self) -> Optional[Tensor]:
+        return self._payload()
 
 
 def _tracks(t: Tensor) -> bool:
@@ -51,8 +58,7 @@ def _derive_operator(sym: str, a: Tensor, b: Tensor, d: int) -> Tensor:
 
 def _broadcast_reduce(sym_op: int, target_like: Tensor, handle: Tensor, error: Tensor, d: int) -> Tensor:
     dev = error.device or target_like.device or handle.device
-    origin = Tensor.of(target_like.dtype, target_like.shape, 0).set_is_virtual(False)
-    dev.store(origin)
+    origin = dev.new_tensor(target_like.dtype, target_like.shape)
     t = F.make_fit([origin, handle, error])
     impl = B.CudaBroadcast(sym_op)
     call = ExecutionCall([t[0], t[1], t[2]], "broadcast-backward", dev, d)
@@ -70,8 +76,7 @@ def _record_operator(sym: str, a: Tensor, b: Tensor, out: Tensor) -> None:
             shape, dtype = t.shape, t.dtype
 
             def action(err, other=other, shape=shape, dtype=dtype):
-                zeros = Tensor.of(dtype, shape, 0).set_is_virtual(False)
-                return F.run_xconv("x»", err, other, zeros)
+                return F.run_xconv("x»", err, other, err.device.new_tensor(dtype, shape))   # the drain: written completely
             parents.append((t, action))
         elif algo == B.BROADCAST or (algo == B.BI_SCALAR_BROADCAST and a.shape != b.shape):
             fa, fb = F.make_fit([a, b]) if a.rank != b.rank else (a, b)
@@ -208,9 +213,7 @@ def evaluate(node, inputs: List[Tensor], do_ad: bool) -> Tensor:
 def _accumulate(t: Tensor, err: Tensor) -> None:
     """TensorImpl.addToGradient (:1275-1300): first error becomes the gradient, later ones are added in place."""
     if t.gradient is None:
-        g = Tensor.of(t.dtype, t.shape, 0).set_is_virtual(False)
-        dev = err.device
-        dev.store(g)
+        g = err.device.new_tensor(t.dtype, t.shape)
         if err.shape != t.shape:
             err = _view_as(err, t.shape)
         F.assign(g, err)
@@ -248,18 +251,20 @@ def backward(result: Tensor, error: Optional[Tensor] = None) -> None:
         raise ValueError("backward needs the result on a CudaDevice")
     if error.device is None:
         dev.store(error)
-    # topological order
-    order, seen = [], set()
-
-    def visit(t: Tensor):
-        if id(t) in seen:
-            return
-        seen.add(id(t))
-        if t.graph_node is not None:
-            for p, _ in t.graph_node.parents:
-                visit(p)
-        order.append(t)
-    visit(result)
+    # topological order: depth first, parents before their children (a stack instead of a recursive closure, which would
+    # hold itself and with it every tensor of the step)
+    order, seen = [], {id(result)}
+    stack = [(result, iter(result.graph_node.parents if result.graph_node is not None else ()))]
+    while stack:
+        t, parents = stack[-1]
+        for p, _ in parents:
+            if id(p) not in seen:
+                seen.add(id(p))
+                stack.append((p, iter(p.graph_node.parents if p.graph_node is not None else ())))
+                break
+        else:
+            order.append(t)
+            stack.pop()
     pending = {id(result): error}
     for t in reversed(order):
         err = pending.pop(id(t), None)

@@ -219,8 +219,7 @@ class CudaSum(ImplementationFor):
         dev = call.device
         src = call.input(0) if call.input(0) is not None else call.input(1)
         src.set_is_virtual(False)
-        out = Tensor.of(src.dtype, (1,), [0])
-        dev.store(out)
+        out = dev.new_tensor(src.dtype, (1,))
         k, c = _cfg(src)
         L.check(L.lib.nk_sum(dev.ctx, nk_dtype(src.dtype), src.rank, src._data.buf, c, out._data.buf, 0), dev.ctx)
         return out
@@ -237,8 +236,7 @@ class CudaReduce(ImplementationFor):
         dev = call.device
         src = call.input(0) if call.input(0) is not None else call.input(1)
         src.set_is_virtual(False)
-        out = Tensor.of(np.int32, (1,), [0])
-        dev.store(out)
+        out = dev.new_tensor(np.int32, (1,))
         k, c = _cfg(src)
         L.check(L.lib.nk_arg_reduce(dev.ctx, self.want_max, nk_dtype(src.dtype), src.rank, src._data.buf, c, out._data.buf, 0), dev.ctx)
         return out

@@ -204,6 +204,14 @@ class CudaDevice:
         L.check(L.lib.nk_write(self.ctx, data.buf, arr.ctypes.data_as(C.c_void_p), 0, 0, arr.size), self.ctx)
         return data
 
+    def new_tensor(self, dtype, shape):
+        """A tensor of this shape on the device whose elements hold nothing yet: for drains a kernel writes completely."""
+        from .tensor import Tensor
+        t = Tensor(dtype, NDConfiguration.of_shape(shape), None)
+        t._attach(self._alloc(t.dtype, t.size), self)
+        self._stored.add(t)
+        return t
+
     # ---- Storage contract ----------------------------------------------------------------------------
     def store(self, tensor) -> "CudaDevice":
         """Storage.store (Storage.java:66) -> AbstractDevice.update(ADDED) -> OpenCLDevice._add (:355-405)."""

@@ -288,3 +288,24 @@ def test_min_and_max_return_the_extreme_item_and_route_the_error_to_its_index(de
     k = base.ndconf.as_inline_array()
     st = L.lib.nk_arg_reduce(device.ctx, 1, L.NK_F32, 2, base._data.buf, k.ctypes.data_as(C.POINTER(C.c_int32)), out._data.buf, 0)
     assert st == L.NK_ERR_BAD_ARG
+
+
+def test_results_of_a_step_are_released_with_their_last_reference(device):
+    """A result knows its graph node, the node must not keep the result: otherwise a training loop's device memory would wait
+    for the interpreter's cycle collector."""
+    import gc
+    a = Tensor.of(np.float32, [12, 20], np.arange(240)).set_rqs_gradient(True).to(device)
+    k = Tensor.of(np.float32, [3, 3], np.arange(9)).set_rqs_gradient(True).to(device)
+    gc.collect()
+    gc.disable()
+    try:
+        n0, t0 = device.number_of_data_objects(), device.number_of_stored()
+        y = Function.of("tanh(i0 x i1) * 2")(a, k)
+        s = y.sum()
+        assert y.graph_node.payload is y and device.number_of_data_objects() > n0
+        s.backward()
+        a.gradient = k.gradient = None
+        del y, s
+        assert device.number_of_data_objects() == n0 and device.number_of_stored() == t0
+    finally:
+        gc.enable()
