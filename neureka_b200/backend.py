@@ -18,6 +18,7 @@ import numpy as np
 
 from . import _lib as L
 from .device import CudaDevice, nk_dtype
+from .ndconf import NDConfiguration
 from .tensor import Tensor
 
 # algorithm names (src/main/java/neureka/backend/main/algorithms/*.java)
@@ -70,6 +71,14 @@ class ExecutionCall:
 
 def _cfg(t: Tensor):
     arr = t.ndconf.as_inline_array()
+    return arr, arr.ctypes.data_as(C.POINTER(C.c_int32))
+
+
+def _cfg_virtual(t: Tensor):
+    """_cfg for an operand that may stay virtual: every index maps to its one element."""
+    if not t.is_virtual:
+        return _cfg(t)
+    arr = NDConfiguration.virtual_of(t.shape).as_inline_array()
     return arr, arr.ctypes.data_as(C.POINTER(C.c_int32))
 
 
@@ -131,10 +140,10 @@ class CudaBiElementwise(ImplementationFor):
             raise ValueError("The element-wise operation requires at least two arguments and one output!")
         dev = call.device
         t0, t1, t2 = call.input(0), call.input(1), call.input(2)
-        for t in (t1, t2):
-            t.set_is_virtual(False)  # CPUBiElementWise.java:59-60
+        # (the reference actualises virtual operands first, CPUBiElementWise.java:59-60; the kernel reads their one element through
+        # a configuration that maps every index to it, which saves filling and re-reading an array of the drain's size)
         dt = _same_type(call, 3)
-        k0, c0 = _cfg(t0); k1, c1 = _cfg(t1); k2, c2 = _cfg(t2)
+        k0, c0 = _cfg(t0); k1, c1 = _cfg_virtual(t1); k2, c2 = _cfg_virtual(t2)
         L.check(L.lib.nk_binary(dev.ctx, self.op, dt, t0.rank, t0._data.buf, c0, t1._data.buf, c1, t2._data.buf, c2, call.deriv_idx), dev.ctx)
         t0.version += 1
         return t0

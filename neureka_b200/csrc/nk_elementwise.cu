@@ -4,6 +4,7 @@
 // Compiled with -fmad=false (see nk_scalarfun.cuh).
 
 #include "nk_ew_kernels.cuh"
+#include "nk_ptx.cuh"
 
 using namespace nkew;
 
@@ -22,6 +23,21 @@ int launch_binary(nk_ctx* ctx, int op, int d, T* out, const T* a, const T* b, co
         }
     }
     return launch_ew<T, 2>(ctx, out, a, b, p, BinF<T, FAMILY>{op, d});
+}
+
+// One term of the backward-broadcast sum, added to 0 like a sum of one element (the sign of a zero differs from the bare term).
+template <class T, int OP, int D> struct TermFix {
+    __device__ __forceinline__ T operator()(T a, T b) const { return T(0) + nkf::bin<0>(OP, D, a, b); }
+};
+template <class T> struct TermF {
+    int op, d;
+    __device__ __forceinline__ T operator()(T a, T b) const { return T(0) + nkf::bin<0>(op, d, a, b); }
+};
+template <class T>
+int launch_term(nk_ctx* ctx, int op, int d, T* out, const T* a, const T* b, const EwPlan& p) {
+    if (op == NK_OP_ADD) return launch_ew<T, 2>(ctx, out, a, b, p, TermFix<T, NK_OP_ADD, 0>{});
+    if (op == NK_OP_MUL_BOTH) return launch_ew<T, 2>(ctx, out, a, b, p, TermFix<T, NK_OP_MUL_BOTH, 0>{});
+    return launch_ew<T, 2>(ctx, out, a, b, p, TermF<T>{op, d});
 }
 
 // ---- broadcast backward: reduction over the dims where the origin is smaller -------------------------
@@ -73,49 +89,66 @@ __global__ void __launch_bounds__(256) nk_broadcast_reduce_kernel(T* __restrict_
     }
 }
 
-// Vectorised variant: the innermost dim is not reduced and all three tensors are unit-stride (the handle may be
-// broadcast) along it, so a thread owns one 128-bit vector of origin elements and every step of its reduction
-// loop is one 128-bit load per operand. The summation order per element is unchanged (lowest reduced dim
-// fastest), hence still bit-identical to the CPU for + - *. OP/D are compile-time for the common operators.
-template <class T, int OP, int D>
-__global__ void __launch_bounds__(256) nk_broadcast_reduce_vec_kernel(T* __restrict__ t0, const T* __restrict__ t1, const T* __restrict__ t2,
-                                                                      RedPlan p, int64_t total_vec, int handle_inner) {
-    using V = typename Vec4<T>::type;
-    constexpr int N = Vec4<T>::N;
+// Vectorised variant: the innermost dim is not reduced and the drain and the origin are unit-stride along it, so a thread owns
+// W neighbouring origin elements (a 128-bit vector, or one element where extents or alignments are odd: lanes still run
+// along contiguous memory) and every step of its reduction loop is one load per operand. What bounds it is the latency of
+// those loads -- the origin is small, so there are few threads -- hence STEPS steps are requested ahead of the (ordered)
+// additions. The summation order per element is unchanged (lowest reduced dim fastest), hence still bit-identical to the
+// CPU for + - *. OP/D are compile-time for the common operators. HMODE: the handle is one value per step (0), runs along with
+// the origin (1), or does not move along the lowest reduced dim at all and is read once per outer step (2: one value, the
+// zero handle of a sum's or difference's backward pass).
+template <class T, int W> struct VecOf { using type = T; };
+template <> struct VecOf<float, 4> { using type = float4; };
+template <> struct VecOf<double, 2> { using type = double2; };
+template <class T, int W, int OP, int D, int HMODE>
+__global__ void __launch_bounds__(128) nk_broadcast_reduce_vec_kernel(T* __restrict__ t0, const T* __restrict__ t1, const T* __restrict__ t2,
+                                                                      RedPlan p, int64_t total_vec) {
+    using V = typename VecOf<T, W>::type;
+    constexpr int STEPS = 8;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t v = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; v < total_vec; v += stride) {
-        int64_t rem = v * N, o0 = p.b0, o1 = p.b1, o2 = p.b2;
+        int64_t rem = v * W, o0 = p.b0, o1 = p.b1, o2 = p.b2;
         for (int k = 0; k < p.rank; k++) {
             int64_t idx = rem / p.odiv[k];
             rem -= idx * p.odiv[k];
             o0 += idx * p.s0[k]; o1 += idx * p.p1[k]; o2 += idx * p.p2[k];
         }
-        T acc[N];
+        T acc[W];
 #pragma unroll
-        for (int k = 0; k < N; k++) acc[k] = T(0);
+        for (int k = 0; k < W; k++) acc[k] = T(0);
         int64_t q[NK_MAX_RANK];
         for (int k = 0; k < p.nred; k++) q[k] = 0;
         const int64_t n0 = p.nred > 0 ? p.rext[0] : 1, a0 = p.nred > 0 ? p.r1[0] : 0, b0 = p.nred > 0 ? p.r2[0] : 0;
         int64_t c1 = o1, c2 = o2;
         while (true) {
-            // lowest reduced dim as a plain loop, 4 steps fetched ahead of the (ordered) additions
-            for (int64_t r = 0; r < n0; r += 4) {
-                T hv[4][N], dv[4][N];
+            const T h_fixed = HMODE == 2 ? t1[c1] : T(0);
+            const T *h_ptr = t1 + c1, *d_ptr = t2 + c2;
+            int64_t r = 0;
+            for (; r + STEPS <= n0; r += STEPS) {
+                T hv[STEPS][W], dv[STEPS][W];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (r + u < n0) {
-                        *reinterpret_cast<V*>(dv[u]) = __ldcs(reinterpret_cast<const V*>(t2 + c2 + (r + u) * b0));
-                        if (handle_inner) *reinterpret_cast<V*>(hv[u]) = __ldg(reinterpret_cast<const V*>(t1 + c1 + (r + u) * a0));
-                        else { T h = t1[c1 + (r + u) * a0]; for (int k = 0; k < N; k++) hv[u][k] = h; }
-                    }
+                for (int u = 0; u < STEPS; u++) {
+                    *reinterpret_cast<V*>(dv[u]) = __ldcs(reinterpret_cast<const V*>(d_ptr));
+                    if (HMODE == 1) *reinterpret_cast<V*>(hv[u]) = __ldg(reinterpret_cast<const V*>(h_ptr));
+                    else if (HMODE == 0) hv[u][0] = __ldg(h_ptr);
+                    d_ptr += b0;
+                    h_ptr += a0;
                 }
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    if (r + u < n0) {
+                for (int u = 0; u < STEPS; u++)
 #pragma unroll
-                        for (int k = 0; k < N; k++) acc[k] += nkf::bin<0>(OP, D, hv[u][k], dv[u][k]);
-                    }
-                }
+                    for (int k = 0; k < W; k++)
+                        acc[k] += nkf::bin<0>(OP, D, HMODE == 1 ? hv[u][k] : HMODE == 0 ? hv[u][0] : h_fixed, dv[u][k]);
+            }
+            for (; r < n0; r++) {
+                T hv[W], dv[W];
+                *reinterpret_cast<V*>(dv) = __ldcs(reinterpret_cast<const V*>(d_ptr));
+                if (HMODE == 1) *reinterpret_cast<V*>(hv) = __ldg(reinterpret_cast<const V*>(h_ptr));
+                else hv[0] = HMODE == 0 ? __ldg(h_ptr) : h_fixed;
+                d_ptr += b0;
+                h_ptr += a0;
+#pragma unroll
+                for (int k = 0; k < W; k++) acc[k] += nkf::bin<0>(OP, D, HMODE == 1 ? hv[k] : hv[0], dv[k]);
             }
             int k = 1;
             for (; k < p.nred; k++) {
@@ -129,24 +162,11 @@ __global__ void __launch_bounds__(256) nk_broadcast_reduce_vec_kernel(T* __restr
     }
 }
 
-template <class T>
-bool try_reduce_vec(nk_ctx* ctx, T* t0, const T* t1, const T* t2, const RedPlan& p, int op, int d, const NkView& v0, int* status) {
-    constexpr int N = Vec4<T>::N;
-    const int last = p.rank - 1;
-    if (p.nred < 1 || !v0.imap_row_major) return false;
-    // innermost dim: kept (not reduced), unit stride in origin and drain, unit or zero stride in the handle
-    if (p.s0[last] != 1 || p.p2[last] != 1 || (p.p1[last] != 1 && p.p1[last] != 0)) return false;
-    if (v0.shape[last] % N) return false;
-    auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    if (!al(t0 + p.b0) || !al(t1 + p.b1) || !al(t2 + p.b2)) return false;
-    for (int k = 0; k < last; k++)
-        if (p.s0[k] % N || p.p1[k] % N || p.p2[k] % N) return false;
-    for (int k = 0; k < p.nred; k++)
-        if (p.r1[k] % N || p.r2[k] % N) return false;
-    const int64_t total_vec = p.total / N;
-    const int hi = p.p1[last] == 1 ? 1 : 0;
-    int block = 256, grid = nk_grid_for(ctx, total_vec, block, 8);
-#define NK_RED(OPC, DC) nk_broadcast_reduce_vec_kernel<T, OPC, DC><<<grid, block, 0, ctx->stream>>>(t0, t1, t2, p, total_vec, hi)
+template <class T, int W, int HMODE>
+bool launch_reduce_vec(nk_ctx* ctx, T* t0, const T* t1, const T* t2, const RedPlan& p, int op, int d, int* status) {
+    const int64_t total_vec = p.total / W;
+    const int block = 128, grid = nk_grid_for(ctx, total_vec, block, 16);
+#define NK_RED(OPC, DC) nk_broadcast_reduce_vec_kernel<T, W, OPC, DC, HMODE><<<grid, block, 0, ctx->stream>>>(t0, t1, t2, p, total_vec)
     if (op == NK_OP_MUL_BOTH) NK_RED(NK_OP_MUL_BOTH, 0);
     else if (op == NK_OP_ADD) NK_RED(NK_OP_ADD, 0);
     else if (op == NK_OP_SUB && d == 0) NK_RED(NK_OP_SUB, 0);
@@ -157,6 +177,32 @@ bool try_reduce_vec(nk_ctx* ctx, T* t0, const T* t1, const T* t2, const RedPlan&
 #undef NK_RED
     *status = nk_after_launch(ctx, "nk_broadcast_reduce_vec_kernel");
     return true;
+}
+
+template <class T>
+bool try_reduce_vec(nk_ctx* ctx, T* t0, const T* t1, const T* t2, const RedPlan& p, int op, int d, const NkView& v0, int* status) {
+    constexpr int N = Vec4<T>::N;
+    const int last = p.rank - 1;
+    if (p.nred < 1 || !v0.imap_row_major) return false;
+    // innermost dim: kept (not reduced), unit stride in origin and drain, unit or zero stride in the handle
+    if (p.s0[last] != 1 || p.p2[last] != 1 || (p.p1[last] != 1 && p.p1[last] != 0)) return false;
+    const bool along = p.p1[last] == 1, fixed = !along && p.r1[0] == 0;
+    // whole 128-bit vectors: extents, strides and addresses allow them for every access (the handle's only if it runs along)
+    auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    bool vec = v0.shape[last] % N == 0 && al(t0 + p.b0) && al(t2 + p.b2) && (!along || al(t1 + p.b1));
+    for (int k = 0; k < last; k++)
+        if (p.s0[k] % N || p.p2[k] % N || (along && p.p1[k] % N)) vec = false;
+    for (int k = 0; k < p.nred; k++)
+        if (p.r2[k] % N || (along && p.r1[k] % N)) vec = false;
+    if (vec) {
+        if (along) return launch_reduce_vec<T, N, 1>(ctx, t0, t1, t2, p, op, d, status);
+        if (fixed) return launch_reduce_vec<T, N, 2>(ctx, t0, t1, t2, p, op, d, status);
+        return launch_reduce_vec<T, N, 0>(ctx, t0, t1, t2, p, op, d, status);
+    }
+    if (v0.shape[last] < 32) return false;   // single elements per lane: worth it where a warp runs along the innermost dim
+    if (along) return launch_reduce_vec<T, 1, 1>(ctx, t0, t1, t2, p, op, d, status);
+    if (fixed) return launch_reduce_vec<T, 1, 2>(ctx, t0, t1, t2, p, op, d, status);
+    return launch_reduce_vec<T, 1, 0>(ctx, t0, t1, t2, p, op, d, status);
 }
 
 // ---- fill with fun(value) ---------------------------------------------------------------------------
@@ -176,31 +222,136 @@ __global__ void __launch_bounds__(256) nk_fill_fun_kernel(T* __restrict__ out, E
 }
 
 // ---- sum: 128-wide tiles, recursively, in CPUSum's order ----------------------------------------------
-// level 0 gathers through the view; one thread adds the 128 elements of its tile in index order.
+// The 128 elements of a tile are added in index order by one lane, so the work is turned through shared memory:
+//   * nk_sum_rows_kernel (contiguous, 16-byte aligned): a warp requests 32 whole tiles with 16-byte asynchronous copies, into rows
+//     padded by 16 bytes, and lane t then adds row t. The copies need no registers: twelve warps' 16 KB each are in flight per
+//     SM. 2^26 F32 elements: 48 us (40 is the floor); sixteen elements of a tile at a time through registers: 170 us.
+//   * nk_sum_tiles_kernel (any view): the same through registers, 16 elements of every tile at a time.
+//   * nk_sum_last_kernel: at most 128 tiles, i.e. the last two levels of any sum (or all of a sum of up to 2^14 elements) in
+//     one CTA: a warp stages a tile, one lane adds it; one lane then adds the tile sums.
+struct SumView {
+    int nd;                       // merged dims
+    int64_t div[NK_MAX_RANK], s[NK_MAX_RANK];
+    int64_t base;
+};
+__device__ __forceinline__ int64_t sum_offset(const SumView& v, int64_t i) {
+    int64_t src = v.base;
+    for (int j = 0; j < v.nd; j++) { const int64_t idx = i / v.div[j]; i -= idx * v.div[j]; src += idx * v.s[j]; }
+    return src;
+}
+template <class T> struct SumRows {
+    static constexpr int VPT = 128 * int(sizeof(T)) / 16;        // 16-byte vectors per tile
+    static constexpr int PITCH = 128 + 16 / int(sizeof(T));      // elements per padded row
+    static constexpr int WARPS = sizeof(T) == 4 ? 4 : 2;
+    static constexpr int SMEM = WARPS * 32 * PITCH * int(sizeof(T));
+};
 template <class T>
-__global__ void __launch_bounds__(128) nk_sum_tiles_kernel(const T* __restrict__ in, EwPlan p, bool through_view, int64_t n,
-                                                           T* __restrict__ out, int64_t n_tiles) {
-    __shared__ T tile[4][128 + 1];
+__global__ void __launch_bounds__(SumRows<T>::WARPS * 32) nk_sum_rows_kernel(const T* __restrict__ in, int64_t n, T* __restrict__ out, int64_t n_tiles) {
+    using C = SumRows<T>;
+    using V = typename Vec4<T>::type;
+    constexpr int N = Vec4<T>::N;
+    extern __shared__ __align__(16) unsigned char sum_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // each warp stages one tile at a time (coalesced), lane 0 then adds it up in order
-    for (int64_t t = int64_t(blockIdx.x) * 4 + warp; t < n_tiles; t += int64_t(gridDim.x) * 4) {
-        const int64_t off = t * 128;
-        const int64_t lim = (off + 128 < n) ? 128 : (n - off);
-        for (int k = lane; k < lim; k += 32) {
-            int64_t i = off + k, src = i;
-            if (through_view) {
-                int64_t rem = i; src = p.b0;
-                for (int j = 0; j < p.nd; j++) { int64_t idx = rem / p.div[j]; rem -= idx * p.div[j]; src += idx * p.s0[j]; }
-            }
-            tile[warp][k] = in[src];
+    T* rows = reinterpret_cast<T*>(sum_smem) + warp * 32 * C::PITCH;
+    const int64_t groups = (n_tiles + 31) / 32;
+    for (int64_t g = int64_t(blockIdx.x) * C::WARPS + warp; g < groups; g += int64_t(gridDim.x) * C::WARPS) {
+        const int64_t first = g * 4096;
+        const int64_t left = n - first;
+        const int count = left < 4096 ? int(left) : 4096;        // elements of this group
+        const int whole = count / N;                             // whole vectors of it; the rest one by one
+        for (int v = lane; v < 32 * C::VPT; v += 32) {
+            T* dst = rows + (v / C::VPT) * C::PITCH + (v % C::VPT) * N;
+            if (v < whole) nk_cp_async_16(dst, in + first + v * N, 16);
+            else
+                for (int e = 0; e < N; e++)
+                    if (v * N + e < count) dst[e] = in[first + v * N + e];
         }
+        nk_cp_async_commit();
+        nk_cp_async_wait<0>();
+        __syncwarp();
+        const int len = count - lane * 128 < 128 ? count - lane * 128 : 128;
+        if (len > 0) {
+            const T* row = rows + lane * C::PITCH;
+            T value = 0;
+            if (len == 128) {
+#pragma unroll 8
+                for (int c = 0; c < 128; c += N) {
+                    T e[N];
+                    *reinterpret_cast<V*>(e) = *reinterpret_cast<const V*>(row + c);
+#pragma unroll
+                    for (int k = 0; k < N; k++) value += e[k];
+                }
+            } else {
+                for (int c = 0; c < len; c++) value += row[c];
+            }
+            out[g * 32 + lane] = value;
+        }
+        __syncwarp();
+    }
+}
+template <class T>
+__global__ void __launch_bounds__(128) nk_sum_tiles_kernel(const T* __restrict__ in, const SumView v, int64_t n, T* __restrict__ out, int64_t n_tiles) {
+    constexpr int C = 16, STEPS = 128 / C, PER = 32 / C;   // elements of a tile per step; lanes 0..C-1 load one tile, C..2C-1 the next
+    __shared__ T stage[4][32][C + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sub = lane / C, col = lane % C;
+    const int64_t groups = (n_tiles + 31) / 32;
+    for (int64_t g = int64_t(blockIdx.x) * 4 + warp; g < groups; g += int64_t(gridDim.x) * 4) {
+        const int64_t first = g * 4096;
+        T val[32 / PER];
+        auto load = [&](int step) {
+#pragma unroll
+            for (int k = 0; k < 32 / PER; k++) {
+                const int64_t i = first + (k * PER + sub) * 128 + step * C + col;
+                val[k] = in[sum_offset(v, i < n ? i : n - 1)];   // past the end: never added
+            }
+        };
+        load(0);
+        const int64_t mine = first + lane * 128;      // this lane's tile
+        const int len = mine >= n ? 0 : (n - mine < 128 ? int(n - mine) : 128);
+        T value = 0;
+        for (int step = 0; step < STEPS; step++) {
+#pragma unroll
+            for (int k = 0; k < 32 / PER; k++) stage[warp][k * PER + sub][col] = val[k];
+            __syncwarp();
+            if (step + 1 < STEPS) load(step + 1);
+            if (len == 128) {
+#pragma unroll
+                for (int c = 0; c < C; c++) value += stage[warp][lane][c];
+            } else {
+                for (int c = 0; c < C; c++)
+                    if (step * C + c < len) value += stage[warp][lane][c];
+            }
+            __syncwarp();
+        }
+        if (len > 0) out[g * 32 + lane] = value;
+    }
+}
+template <class T>
+__global__ void __launch_bounds__(1024) nk_sum_last_kernel(const T* __restrict__ in, const SumView v, int n, T* __restrict__ out) {
+    __shared__ T tile[32][128 + 1];
+    __shared__ T part[128];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_tiles = (n + 127) / 128;
+    for (int t = warp; t < n_tiles; t += 32) {
+        const int off = t * 128;
+        const int lim = off + 128 < n ? 128 : n - off;
+        for (int k = lane; k < lim; k += 32) tile[warp][k] = in[sum_offset(v, off + k)];
         __syncwarp();
         if (lane == 0) {
             T value = 0;
             for (int k = 0; k < lim; k++) value += tile[warp][k];
-            out[t] = value;
+            part[t] = value;
         }
         __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // a single tile is the result; several are one more tile, added in order from 0
+        T value = 0;
+        if (n_tiles == 1) value = part[0];
+        else for (int k = 0; k < n_tiles; k++) value += part[k];
+        *out = value;
     }
 }
 
@@ -265,6 +416,18 @@ extern "C" int nk_broadcast(nk_ctx* ctx, int32_t op, int32_t dtype, int32_t rank
             p.nred++;
         }
     }
+    if (p.nred == 0) {
+        // nothing is summed (the origin has the error's shape): an elementwise pass, with the reduction's 0 + term
+        bool f1[NK_MAX_RANK], f2[NK_MAX_RANK];
+        for (int k = 0; k < rank; k++) {
+            f1[k] = v0.shape[k] == v1.shape[k];
+            f2[k] = !f1[k] || v2.shape[k] != 1;
+        }
+        EwPlan e;
+        make_plan(v0, &v1, f1, &v2, f2, &e);
+        if (dtype == NK_F32) return launch_term<float>(ctx, op, d, data_of<float>(drn), data_of<float>(a), data_of<float>(b), e);
+        return launch_term<double>(ctx, op, d, data_of<double>(drn), data_of<double>(a), data_of<double>(b), e);
+    }
     {
         int vst = NK_OK;
         bool done = (dtype == NK_F32) ? try_reduce_vec<float>(ctx, data_of<float>(drn), data_of<float>(a), data_of<float>(b), p, op, d, v0, &vst)
@@ -317,39 +480,47 @@ extern "C" int nk_fill_fun(nk_ctx* ctx, int32_t fun, int32_t dtype, int32_t rank
 
 template <class T>
 static int sum_impl(nk_ctx* ctx, const T* in, const EwPlan& p, int64_t n, T* out_elem) {
-    // level sizes: n -> ceil(n/128) -> ... -> 1 ; ping-pong inside the ctx scratch block
-    int64_t n1 = (n + 127) / 128;
-    int64_t n2 = (n1 + 127) / 128;
-    void* scratch = nullptr;
-    int st = nk_scratch(ctx, size_t(n1 + n2 + 2) * sizeof(T), &scratch);
-    if (st) return st;
-    T* bufA = reinterpret_cast<T*>(scratch);
-    T* bufB = bufA + n1 + 1;
+    // levels n -> ceil(n / 128) -> ... ping-pong inside the ctx scratch block, until one CTA can do the rest
+    SumView v;
+    memset(&v, 0, sizeof(v));
+    v.nd = p.nd;
+    v.base = p.b0;
+    for (int k = 0; k < p.nd; k++) { v.div[k] = p.div[k]; v.s[k] = p.s0[k]; }
+    bool rows = p.nd == 1 && p.row_major && p.s0[0] == 1 && aligned16(in + p.b0);
+    if (rows) { in += p.b0; v.base = 0; }
+    T *bufA = nullptr, *bufB = nullptr;
+    if (n > 16384) {
+        const int64_t n1 = (n + 127) / 128, n2 = (n1 + 127) / 128;
+        void* scratch = nullptr;
+        int st = nk_scratch(ctx, size_t(n1 + n2 + 16) * sizeof(T), &scratch);
+        if (st) return st;
+        bufA = reinterpret_cast<T*>(scratch);
+        bufB = bufA + ((n1 + 7) / 8) * 8;   // 16-byte aligned like bufA
+        NK_CUDA(ctx, cudaFuncSetAttribute(nk_sum_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SumRows<T>::SMEM));
+    }
     const T* src = in;
     int64_t cur = n;
-    bool through_view = true;
     T* dst = bufA;
-    if (cur == 1) {
-        // CPUSum returns the input itself for a single element
-        nk_sum_tiles_kernel<T><<<1, 128, 0, ctx->stream>>>(src, p, true, 1, out_elem, 1);
-        return nk_after_launch(ctx, "nk_sum_tiles_kernel");
-    }
-    while (true) {
-        int64_t tiles = (cur + 127) / 128;
-        T* target = (tiles == 1) ? out_elem : dst;
-        int64_t want = (tiles + 3) / 4;
-        int64_t cap = int64_t(ctx->prop.multiProcessorCount) * 16;
-        int grid = int(want < cap ? want : cap);
-        nk_sum_tiles_kernel<T><<<grid, 128, 0, ctx->stream>>>(src, p, through_view, cur, target, tiles);
-        st = nk_after_launch(ctx, "nk_sum_tiles_kernel");
+    while (cur > 16384) {
+        const int64_t tiles = (cur + 127) / 128;
+        if (rows) {
+            using C = SumRows<T>;
+            nk_sum_rows_kernel<T><<<nk_grid_for(ctx, (tiles + 31) / 32, C::WARPS, 12), C::WARPS * 32, C::SMEM, ctx->stream>>>(src, cur, dst, tiles);
+        } else {
+            nk_sum_tiles_kernel<T><<<nk_grid_for(ctx, (tiles + 31) / 32, 4, 16), 128, 0, ctx->stream>>>(src, v, cur, dst, tiles);
+        }
+        const int st = nk_after_launch(ctx, "nk_sum_tiles_kernel");
         if (st) return st;
-        if (tiles == 1) break;
-        src = target;
-        through_view = false;
+        src = dst;
+        rows = true;   // the next levels are dense
+        v.nd = 1;
+        v.base = 0;
+        v.div[0] = v.s[0] = 1;
         cur = tiles;
         dst = (dst == bufA) ? bufB : bufA;
     }
-    return NK_OK;
+    nk_sum_last_kernel<T><<<1, 1024, 0, ctx->stream>>>(src, v, int(cur), out_elem);
+    return nk_after_launch(ctx, "nk_sum_last_kernel");
 }
 
 extern "C" int nk_sum(nk_ctx* ctx, int32_t dtype, int32_t rank, nk_buf* src, const int32_t* cfg, nk_buf* out, int64_t out_index) {

@@ -279,7 +279,125 @@ __global__ void __launch_bounds__(256) nk_ew_rows_kernel(T* __restrict__ out, co
     }
 }
 
-// ---- kernel 3: flat, any view -----------------------------------------------------------------------
+// ---- kernel 3: tiles, an operand whose contiguous direction is another dim than the drain's ----------------------------
+// A transposed operand read in the drain's order touches one 32-byte sector per 4-byte element. Here a CTA takes a 32 x 32 tile
+// of (dim t, innermost dim): the transposed operands (bit mask) are read along t, where they are contiguous, and turned in
+// shared memory; everything else is read and written along the innermost dim. The other dims are the grid's z index.
+struct TileWalk {
+    int t, nrest;                 // the operands' contiguous dim; number of remaining dims
+    int64_t ext_t, ext_l;
+    int64_t tiles_l;
+    int64_t s0t, s1t, s2t, s1l, s2l;   // strides along t and the innermost dim (the drain's innermost stride is 1)
+    int64_t rext[NK_MAX_RANK], r0[NK_MAX_RANK], r1[NK_MAX_RANK], r2[NK_MAX_RANK];   // remaining dims, fastest first
+    int turn1, turn2;             // which sources go through shared memory
+};
+template <class T, int NIN, class F>
+__global__ void __launch_bounds__(256) nk_ew_tiles_kernel(T* __restrict__ out, const T* __restrict__ a, const T* __restrict__ b,
+                                                          int64_t b0, int64_t b1, int64_t b2, TileWalk w, F f) {
+    __shared__ T ta[32][33], tb[NIN == 2 ? 32 : 1][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    int64_t rem = blockIdx.y, o0 = b0, o1 = b1, o2 = b2;
+    for (int k = 0; k < w.nrest; k++) {
+        const int64_t idx = rem % w.rext[k];
+        rem /= w.rext[k];
+        o0 += idx * w.r0[k]; o1 += idx * w.r1[k]; o2 += idx * w.r2[k];
+    }
+    const int64_t l0 = (blockIdx.x % w.tiles_l) * 32, t0 = (blockIdx.x / w.tiles_l) * 32;
+    // turned sources: lanes run along t
+    if (w.turn1) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t t = t0 + tx, l = l0 + ty + 8 * i;
+            if (t < w.ext_t && l < w.ext_l) ta[ty + 8 * i][tx] = a[o1 + t * w.s1t + l * w.s1l];
+        }
+    }
+    if (NIN == 2 && w.turn2) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int64_t t = t0 + tx, l = l0 + ty + 8 * i;
+            if (t < w.ext_t && l < w.ext_l) tb[ty + 8 * i][tx] = b[o2 + t * w.s2t + l * w.s2l];
+        }
+    }
+    const int64_t l = l0 + tx;
+    T av[4], bv[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int64_t t = t0 + ty + 8 * i;
+        const bool ok = t < w.ext_t && l < w.ext_l;
+        av[i] = !w.turn1 && ok ? a[o1 + t * w.s1t + l * w.s1l] : T(0);
+        bv[i] = NIN == 2 && !w.turn2 && ok ? b[o2 + t * w.s2t + l * w.s2l] : T(0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int64_t t = t0 + ty + 8 * i;
+        if (t >= w.ext_t || l >= w.ext_l) continue;
+        if (w.turn1) av[i] = ta[tx][ty + 8 * i];
+        if (NIN == 2 && w.turn2) bv[i] = tb[tx][ty + 8 * i];
+        out[o0 + t * w.s0t + l] = f(av[i], bv[i]);
+    }
+}
+
+// ---- kernel 4: flat, row-major views of up to 2^31 elements ----------------------------------------------------------
+// Odd row lengths and unaligned views. The flat index is taken apart with multiply-high divisions by the (merged) extents;
+// four elements per thread, a grid apart, so that neighbouring lanes stay on neighbouring elements and four loads per
+// operand are in flight.
+struct FastDiv {
+    unsigned d, m, l;
+};
+inline FastDiv fast_div(unsigned d) {   // exact for dividends below 2^31
+    FastDiv r;
+    r.d = d;
+    r.l = 0;
+    while ((uint64_t(1) << r.l) < d) r.l++;
+    r.m = unsigned((((uint64_t(1) << r.l) - d) << 32) / d + 1);
+    return r;
+}
+__device__ __forceinline__ unsigned fast_quot(unsigned n, const FastDiv& f) { return (__umulhi(f.m, n) + n) >> f.l; }
+struct Flat32 {
+    unsigned total;
+    FastDiv ext[3];               // extents, outermost first; entry 0 is never divided by
+    int64_t s0[3], s1[3], s2[3];
+    int64_t b0, b1, b2;
+};
+template <class T, int NIN, class F, int ND>
+__global__ void __launch_bounds__(256) nk_ew_flat32_kernel(T* __restrict__ out, const T* __restrict__ a, const T* __restrict__ b,
+                                                           const Flat32 p, F f) {
+    constexpr int U = 4;
+    const unsigned stride = gridDim.x * blockDim.x;
+    for (unsigned base = blockIdx.x * blockDim.x + threadIdx.x; base < p.total; base += U * stride) {   // base < 2^31, U * stride < 2^31
+        int64_t o0[U];
+        T av[U], bv[U];
+        bool ok[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const unsigned i = base + u * stride;
+            ok[u] = i < p.total;
+            unsigned rem = ok[u] ? i : 0;
+            int64_t o1 = p.b1, o2 = p.b2;
+            o0[u] = p.b0;
+#pragma unroll
+            for (int k = ND - 1; k >= 0; k--) {
+                unsigned idx = rem;
+                if (k > 0) {
+                    const unsigned q = fast_quot(rem, p.ext[k]);
+                    idx = rem - q * p.ext[k].d;
+                    rem = q;
+                }
+                o0[u] += idx * p.s0[k];
+                o1 += idx * p.s1[k];
+                if (NIN == 2) o2 += idx * p.s2[k];
+            }
+            av[u] = a[o1];
+            bv[u] = NIN == 2 ? b[o2] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (ok[u]) out[o0[u]] = f(av[u], bv[u]);
+    }
+}
+
+// ---- kernel 5: flat, any view -----------------------------------------------------------------------
 template <class T, int NIN, class F>
 __global__ void __launch_bounds__(256) nk_ew_flat_kernel(T* __restrict__ out, const T* __restrict__ a, const T* __restrict__ b,
                                                          EwPlan p, F f) {
@@ -355,6 +473,50 @@ int launch_ew(nk_ctx* ctx, T* out, const T* a, const T* b, const EwPlan& p_in, F
             else nk_ew_rows_kernel<T, NIN, F, 2><<<unsigned(grid), block, 0, ctx->stream>>>(out, a, b, p, rw, f);
             return nk_after_launch(ctx, "nk_ew_rows_kernel");
         }
+    }
+    // a source that is contiguous along another dim than the drain, which it shares with the drain
+    if (p.row_major && p.nd >= 2 && p.s0[last] == 1 && p.ext[last] >= 32) {
+        auto strided = [&](int64_t s) { return s != 0 && s != 1; };
+        const bool want1 = strided(p.s1[last]), want2 = NIN == 2 && strided(p.s2[last]);
+        int t = -1;
+        for (int k = 0; k < last && (want1 || want2); k++)
+            if (p.ext[k] >= 32 && ((want1 && p.s1[k] == 1) || (want2 && p.s2[k] == 1))) t = k;
+        if (t >= 0) {
+            TileWalk w;
+            memset(&w, 0, sizeof(w));
+            w.t = t;
+            w.ext_t = p.ext[t]; w.ext_l = p.ext[last];
+            w.tiles_l = (w.ext_l + 31) / 32;
+            w.s0t = p.s0[t]; w.s1t = p.s1[t]; w.s2t = p.s2[t]; w.s1l = p.s1[last]; w.s2l = p.s2[last];
+            w.turn1 = want1 && p.s1[t] == 1; w.turn2 = want2 && p.s2[t] == 1;
+            int64_t rest = 1;
+            for (int k = last - 1; k >= 0; k--) {
+                if (k == t) continue;
+                w.rext[w.nrest] = p.ext[k]; w.r0[w.nrest] = p.s0[k]; w.r1[w.nrest] = p.s1[k]; w.r2[w.nrest] = p.s2[k];
+                w.nrest++;
+                rest *= p.ext[k];
+            }
+            const int64_t tiles = w.tiles_l * ((w.ext_t + 31) / 32);
+            if (tiles <= 0x7fffffff && rest <= 65535) {
+                nk_ew_tiles_kernel<T, NIN, F><<<dim3(unsigned(tiles), unsigned(rest)), block, 0, ctx->stream>>>(out, a, b, p.b0, p.b1, p.b2, w, f);
+                return nk_after_launch(ctx, "nk_ew_tiles_kernel");
+            }
+        }
+    }
+    if (p.row_major && p.nd <= 3 && p.total < (int64_t(1) << 31)) {
+        Flat32 q;
+        memset(&q, 0, sizeof(q));
+        q.total = unsigned(p.total);
+        for (int k = 0; k < p.nd; k++) {
+            q.ext[k] = fast_div(unsigned(p.ext[k]));
+            q.s0[k] = p.s0[k]; q.s1[k] = p.s1[k]; q.s2[k] = p.s2[k];
+        }
+        q.b0 = p.b0; q.b1 = p.b1; q.b2 = p.b2;
+        const int g = nk_grid_for(ctx, (p.total + 3) / 4, block, 8);
+        if (p.nd == 1) nk_ew_flat32_kernel<T, NIN, F, 1><<<g, block, 0, ctx->stream>>>(out, a, b, q, f);
+        else if (p.nd == 2) nk_ew_flat32_kernel<T, NIN, F, 2><<<g, block, 0, ctx->stream>>>(out, a, b, q, f);
+        else nk_ew_flat32_kernel<T, NIN, F, 3><<<g, block, 0, ctx->stream>>>(out, a, b, q, f);
+        return nk_after_launch(ctx, "nk_ew_flat32_kernel");
     }
     int grid = nk_grid_for(ctx, p.total, block, 16);
     nk_ew_flat_kernel<T, NIN, F><<<grid, block, 0, ctx->stream>>>(out, a, b, p, f);

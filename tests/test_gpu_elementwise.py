@@ -254,3 +254,60 @@ def test_permuted_slices_as_operands(device, oracle):
             for j in range(3):
                 ref[c, i, j] = np.sum(host[c, i:i + 3, j:j + 3].astype(np.float64) * k.numpy()[0].astype(np.float64))
     assert np.abs(y.numpy() - ref).max() <= 1e-5 * np.abs(ref).max() * 4
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [127, 4096, 16385, 32 * 128 * 5 + 3, (1 << 21) + 77])
+def test_sums_at_the_edges_of_tiles_and_groups(device, oracle, dt, n):
+    """One CTA up to 2^14 elements; whole and partial groups of 32 tiles through 16-byte copies, from an aligned and (one element
+    further) an unaligned start, and through a view with gaps: always CPUSum's order, hence its bits."""
+    rng = np.random.default_rng(n)
+    host = rng.standard_normal(2 * n + 1).astype(dt)
+    S, O = DevArray(device, host), DevArray(device, np.zeros(1, dtype=dt))
+    parent = ND.of_shape([2 * n + 1])
+    for conf, items in ((parent.sliced([n], [0], [1]), host[:n]), (parent.sliced([n], [1], [1]), host[1:n + 1]),
+                        (parent.sliced([n], [1], [2]), host[1::2][:n])):
+        k, p = cfgp(conf)
+        L.check(L.lib.nk_sum(device.ctx, S.nk_dtype, 1, S.buf, p, O.buf, 0), device.ctx)
+        assert O.read()[0] == dt(oracle.cpu_sum(np.ascontiguousarray(items)))
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("op,d", [("*", 0), ("+", 0), ("-", 0), ("-", 1)])
+def test_broadcast_backward_at_odd_extents_and_with_a_one_element_handle(device, oracle, dt, op, d):
+    """The reduction with one element per lane (odd inner extents), step counts around the number of steps fetched ahead, two
+    reduced dims, and a handle that is one element standing for a whole shape."""
+    rng = np.random.default_rng(53)
+    for s0, s1, s2 in (([5, 1, 33], [1, 8, 33], [5, 8, 33]), ([5, 1, 33], [1, 9, 33], [5, 9, 33]), ([1, 6, 35], [17, 1, 35], [17, 6, 35]),
+                       ([1, 1, 64], [7, 9, 64], [7, 9, 64]), ([3, 1, 64], [1, 23, 1], [3, 23, 64]), ([4, 7, 33], [1, 7, 33], [4, 7, 33])):
+        dr = _inputs(rng, int(np.prod(s2)), dt)
+        c0, c1, c2 = ND.of_shape(s0), ND.of_shape(s1), ND.of_shape(s2)
+        h = _inputs(rng, c1.size, dt)
+        for handle, conf in ((h, c1), (np.zeros(1, dtype=dt), ND.virtual_of(s1))):
+            full = handle if handle.size > 1 else np.zeros(c1.size, dtype=dt)
+            ref = np.zeros(c0.size, dtype=dt)
+            oracle.broadcast(op, ref, c0.as_inline_array(), full, c1.as_inline_array(), dr, c2.as_inline_array(), d=d)
+            got = gpu_call3(L.lib.nk_broadcast, device, L.OPS[op], np.zeros(c0.size, dtype=dt), c0, handle, conf, dr, c2, d=d)
+            assert np.array_equal(got, ref), (op, s0, handle.size)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("shape", [(32, 32), (33, 95), (70, 32), (3, 65, 41), (2, 40, 3, 37)])
+def test_transposed_operands_and_odd_rows(device, dt, shape):
+    """Operands that are contiguous along another dim than the drain (one, the other, both), at sizes around the 32 x 32 tiles,
+    and odd dense rows against a row vector: one rounding per element, compared exactly."""
+    rng = np.random.default_rng(59)
+    rank = len(shape)
+    swap = list(range(rank)); swap[0], swap[-1] = swap[-1], swap[0]
+    parent = [shape[i] for i in swap]
+    dense, turned = ND.of_shape(shape), ND.of_shape(parent).reshaped(swap)
+    a, b = (_inputs(rng, dense.size, dt) for _ in range(2))
+    av, bv = a.reshape(shape), b.reshape(shape)
+    at, bt = a.reshape(parent).transpose(swap), b.reshape(parent).transpose(swap)
+    for ca, cb, x, y in ((dense, turned, av, bt), (turned, dense, at, bv), (turned, turned, at, bt)):
+        got = gpu_call3(L.lib.nk_binary, device, L.OPS["*"], np.zeros(dense.size, dtype=dt), dense, a, ca, b, cb)
+        assert np.array_equal(got.reshape(shape), x * y)
+    row = _inputs(rng, shape[-1], dt)
+    cr = ND.of_shape([1] * (rank - 1) + [shape[-1]])
+    got = gpu_call3(L.lib.nk_broadcast, device, L.OPS["-"], np.zeros(dense.size, dtype=dt), dense, a, dense, row, cr)
+    assert np.array_equal(got.reshape(shape), av - row)
