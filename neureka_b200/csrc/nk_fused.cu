@@ -52,6 +52,17 @@ struct FusedFlat {
     long long div[NK_MAX_RANK], s0[NK_MAX_RANK], s[NK_FUSED_MAX_IN][NK_MAX_RANK];
 };
 
+// Forward, views of up to 2^31 elements in up to three merged dims (missing ones in front, extent 1): the decode divides by
+// multiply-high (d, m, l as in the elementwise family's FastDiv).
+struct FusedFlat32 {
+    void* out;
+    const void* in[NK_FUSED_MAX_IN];
+    long long b0, b[NK_FUSED_MAX_IN];
+    unsigned total;
+    unsigned d[3], m[3], l[3];
+    long long s0[3], s[NK_FUSED_MAX_IN][3];
+};
+
 // Backward: one thread per vector of target elements; sums over the dims the target is broadcast along.
 struct FusedGrad {
     void* out;
@@ -70,6 +81,7 @@ struct nk_fused {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t kernel = nullptr;        // forward: flat form; backward: the gradient kernel
     cudaKernel_t rows1 = nullptr, rows2 = nullptr;   // forward, rows form with one / two outer dims
+    cudaKernel_t flat32 = nullptr;                   // forward, flat form of up to 2^31 elements in three merged dims
     int grad_target = -1;                 // >= 0: a backward operation for this input
     int n_leaves = 0;
     int dtype = NK_F32;
@@ -163,6 +175,14 @@ struct FusedFlat {
     long long total;
     int nd;
     long long div[NK_MAX_RANK], s0[NK_MAX_RANK], s[NK_FUSED_MAX_IN][NK_MAX_RANK];
+};
+struct FusedFlat32 {
+    void* out;
+    const void* in[NK_FUSED_MAX_IN];
+    long long b0, b[NK_FUSED_MAX_IN];
+    unsigned total;
+    unsigned d[3], m[3], l[3];
+    long long s0[3], s[NK_FUSED_MAX_IN][3];
 };
 
 __device__ __forceinline__ T nk_expr(T x0, T x1, T x2, T x3, T x4, T x5) { return NK_EXPR; }
@@ -280,6 +300,52 @@ __device__ __forceinline__ void nk_fused_rows(const FusedRows& a) {
 extern "C" __global__ void __launch_bounds__(256, NK_MIN_CTAS) nk_fused_rows1(const FusedRows a) { nk_fused_rows<1>(a); }
 extern "C" __global__ void __launch_bounds__(256, NK_MIN_CTAS) nk_fused_rows2(const FusedRows a) { nk_fused_rows<2>(a); }
 
+// Flat form for odd row lengths and unaligned views: four elements per thread, a grid apart (neighbouring lanes on
+// neighbouring elements, four loads per operand in flight), two 32-bit multiply-high divisions per element instead of
+// 64-bit ones.
+extern "C" __global__ void __launch_bounds__(256) nk_fused_flat32(const FusedFlat32 a) {
+    T* out = reinterpret_cast<T*>(a.out);
+    const unsigned stride = gridDim.x * blockDim.x;
+    for (unsigned base = blockIdx.x * blockDim.x + threadIdx.x; base < a.total; base += 4 * stride) {
+        T x[4][NK_NIN];
+        long long o0[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            unsigned rem = base + u * stride;
+            if (rem >= a.total) rem = 0;
+            long long oi[NK_NIN];
+#pragma unroll
+            for (int j = 0; j < NK_NIN; j++) oi[j] = a.b[j];
+            o0[u] = a.b0;
+#pragma unroll
+            for (int k = 2; k >= 0; k--) {
+                unsigned idx = rem;
+                if (k > 0) {
+                    const unsigned q = (__umulhi(a.m[k], rem) + rem) >> a.l[k];
+                    idx = rem - q * a.d[k];
+                    rem = q;
+                }
+                o0[u] += idx * a.s0[k];
+#pragma unroll
+                for (int j = 0; j < NK_NIN; j++) oi[j] += idx * a.s[j][k];
+            }
+#pragma unroll
+            for (int j = 0; j < NK_NIN; j++) x[u][j] = __ldg(reinterpret_cast<const T*>(a.in[j]) + oi[j]);
+        }
+        T res[4];
+        bool rare = false;
+#pragma unroll
+        for (int u = 0; u < 4; u++) res[u] = nk_eval_fast(x[u], rare);
+        if (rare) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) res[u] = nk_eval(x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (base + u * stride < a.total) out[o0[u]] = res[u];
+    }
+}
+
 extern "C" __global__ void __launch_bounds__(256) nk_fused_kernel(const FusedFlat a) {
     T* out = reinterpret_cast<T*>(a.out);
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -322,7 +388,11 @@ struct FusedGrad {
 };
 __device__ __forceinline__ void nk_terms(T e, T x0, T x1, T x2, T x3, T x4, T x5, T* term) { NK_TERMS }
 
-template <int VEC>
+// Two forms. VEC = a 128-bit vector of target elements per thread and one position at a time: nothing (or next to nothing)
+// is summed. STEPS > 1: one element per thread, the lowest reduced dim walked STEPS positions at a time with all their
+// operands requested before the first (ordered) addition -- a target has few elements, so few threads have to keep the memory
+// system busy, and neighbouring lanes still read neighbouring elements.
+template <int VEC, int STEPS>
 __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
     T* out = reinterpret_cast<T*>(a.out);
     const T* err = reinterpret_cast<const T*>(a.err);
@@ -344,7 +414,7 @@ __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
         for (int l = 0; l < NK_NLEAF; l++)
 #pragma unroll
             for (int e = 0; e < VEC; e++) acc[l][e] = T(0);
-        T x[NK_NIN + 1][VEC];   // [NK_NIN] is the error
+        T x[NK_NIN + 1][VEC] = {};   // operands that stay; [NK_NIN] is the error
         auto fetch = [&](int j, const T* p, bool streams) {
             if (VEC > 1 && streams) *reinterpret_cast<V*>(x[j]) = *reinterpret_cast<const V*>(p);
             else { const T s = p[0];
@@ -356,22 +426,52 @@ __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
         for (int j = 0; j < NK_NIN; j++)
             if ((a.invariant_mask >> j) & 1u) fetch(j, reinterpret_cast<const T*>(a.in[j]) + oi[j], (a.stream_mask >> j) & 1u);
         if ((a.invariant_mask >> 6) & 1u) fetch(NK_NIN, err + oe, (a.stream_mask >> 6) & 1u);
+        const long long n0 = a.nr > 0 ? a.rext[0] : 1, e0 = a.nr > 0 ? a.rse[0] : 0;
+        long long i0[NK_NIN];
+#pragma unroll
+        for (int j = 0; j < NK_NIN; j++) i0[j] = a.nr > 0 ? a.rs[j][0] : 0;
         long long q[NK_MAX_RANK];
         for (int k = 0; k < a.nr; k++) q[k] = 0;
-        while (true) {
-#pragma unroll
-            for (int j = 0; j < NK_NIN; j++)
-                if (!((a.invariant_mask >> j) & 1u)) fetch(j, reinterpret_cast<const T*>(a.in[j]) + oi[j], (a.stream_mask >> j) & 1u);
-            if (!((a.invariant_mask >> 6) & 1u)) fetch(NK_NIN, err + oe, (a.stream_mask >> 6) & 1u);
+        // (positions past the end are evaluated and not added: a branch per step would keep the steps' arithmetic from overlapping)
+        auto step = [&](const T (*xs)[VEC], bool add) {
 #pragma unroll
             for (int e = 0; e < VEC; e++) {
                 T term[NK_NLEAF];
-                nk_terms(x[NK_NIN][e], x[0][e], x[NK_NIN > 1 ? 1 : 0][e], x[NK_NIN > 2 ? 2 : 0][e], x[NK_NIN > 3 ? 3 : 0][e],
-                         x[NK_NIN > 4 ? 4 : 0][e], x[NK_NIN > 5 ? 5 : 0][e], term);
+                nk_terms(xs[NK_NIN][e], xs[0][e], xs[NK_NIN > 1 ? 1 : 0][e], xs[NK_NIN > 2 ? 2 : 0][e], xs[NK_NIN > 3 ? 3 : 0][e],
+                         xs[NK_NIN > 4 ? 4 : 0][e], xs[NK_NIN > 5 ? 5 : 0][e], term);
 #pragma unroll
-                for (int l = 0; l < NK_NLEAF; l++) acc[l][e] += term[l];
+                for (int l = 0; l < NK_NLEAF; l++) {
+                    const T sum = acc[l][e] + term[l];
+                    acc[l][e] = add ? sum : acc[l][e];
+                }
             }
-            int k = 0;
+        };
+        auto load = [&](T (*xs)[VEC], long long r) {   // the operands of position r of the lowest reduced dim
+#pragma unroll
+            for (int j = 0; j <= NK_NIN; j++) {
+                const unsigned bit = j < NK_NIN ? j : 6;
+                const T* p = j < NK_NIN ? reinterpret_cast<const T*>(a.in[j < NK_NIN ? j : 0]) + oi[j < NK_NIN ? j : 0] + r * i0[j < NK_NIN ? j : 0] : err + oe + r * e0;
+                if ((a.invariant_mask >> bit) & 1u) {
+#pragma unroll
+                    for (int e = 0; e < VEC; e++) xs[j][e] = x[j][e];
+                } else if (VEC > 1 && ((a.stream_mask >> bit) & 1u)) {
+                    *reinterpret_cast<V*>(xs[j]) = __ldg(reinterpret_cast<const V*>(p));
+                } else {
+                    const T s = __ldg(p);
+#pragma unroll
+                    for (int e = 0; e < VEC; e++) xs[j][e] = s;
+                }
+            }
+        };
+        while (true) {
+            for (long long r = 0; r < n0; r += STEPS) {
+                T xs[STEPS][NK_NIN + 1][VEC];
+#pragma unroll
+                for (int u = 0; u < STEPS; u++) load(xs[u], r + u < n0 ? r + u : n0 - 1);
+#pragma unroll
+                for (int u = 0; u < STEPS; u++) step(xs[u], r + u < n0);
+            }
+            int k = 1;
             for (; k < a.nr; k++) {
                 q[k]++; oe += a.rse[k];
 #pragma unroll
@@ -396,7 +496,7 @@ __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
     }
 }
 extern "C" __global__ void __launch_bounds__(256) nk_fused_grad_kernel(const FusedGrad a) {
-    if (a.vec > 1) nk_grad_body<VECW>(a); else nk_grad_body<1>(a);
+    if (a.vec > 1) nk_grad_body<VECW, 1>(a); else nk_grad_body<1, 8>(a);
 }
 )NKSRC";
 
@@ -474,6 +574,7 @@ extern "C" int nk_fused_compile(nk_ctx* ctx, int32_t dtype, int32_t n_inputs, co
     cudaError_t e = cudaLibraryGetKernel(&f->kernel, f->lib, "nk_fused_kernel");
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&f->rows1, f->lib, "nk_fused_rows1");
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&f->rows2, f->lib, "nk_fused_rows2");
+    if (e == cudaSuccess) e = cudaLibraryGetKernel(&f->flat32, f->lib, "nk_fused_flat32");
     if (e != cudaSuccess) {
         cudaLibraryUnload(f->lib);
         delete f;
@@ -605,6 +706,28 @@ extern "C" int nk_fused_run(nk_ctx* ctx, nk_fused* f, int32_t rank, nk_buf* drn,
         return nk_after_launch(ctx, "nk_fused_rows_kernel");
     }
     // ---- any other view: per-element decode ----
+    int64_t total = 1;
+    for (int k = 0; k < nd; k++) total *= ext[k];
+    if (nd <= 3 && total < (int64_t(1) << 31)) {
+        FusedFlat32 q;
+        memset(&q, 0, sizeof(q));
+        q.out = drn->ptr;
+        q.b0 = v0.base;
+        q.total = unsigned(total);
+        for (int k = 0; k < 3; k++) {
+            const int from = k - (3 - nd);
+            const unsigned d = from >= 0 ? unsigned(ext[from]) : 1u;
+            q.d[k] = d;
+            while ((uint64_t(1) << q.l[k]) < d) q.l[k]++;
+            q.m[k] = unsigned((((uint64_t(1) << q.l[k]) - d) << 32) / d + 1);
+            q.s0[k] = from >= 0 ? m0[from] : 0;
+            for (int j = 0; j < f->n_in; j++) q.s[j][k] = from >= 0 ? m[j][from] : 0;
+        }
+        for (int j = 0; j < f->n_in; j++) { q.in[j] = srcs[j]->ptr; q.b[j] = v[j].base; }
+        void* params[] = {&q};
+        NK_CUDA(ctx, cudaLaunchKernel(reinterpret_cast<const void*>(f->flat32), dim3(unsigned(nk_grid_for(ctx, (total + 3) / 4, 256, 8))), dim3(256), params, 0, ctx->stream));
+        return nk_after_launch(ctx, "nk_fused_kernel");
+    }
     FusedFlat a;
     memset(&a, 0, sizeof(a));
     a.out = drn->ptr;
@@ -701,6 +824,8 @@ extern "C" int nk_fused_run_grad(nk_ctx* ctx, nk_fused* f, int32_t rank, nk_buf*
         for (int j = 0; j < f->n_in && vec; j++) vec = lane_ok(a.ks[j][n], srcs[j]->ptr, v[j].base, a.ks[j], a.rs[j], 1u << j);
         for (int q = 0; q < n && vec; q++) vec = a.ks0[q] % W == 0;
     }
+    // fewer than four positions of the lowest reduced dim: whole vectors (where possible); otherwise one element per thread
+    if (a.nr > 0 && a.rext[0] >= 4) vec = false;
     if (!vec) a.stream_mask = 0;
     a.vec = vec ? W : 1;
     int64_t d = 1;

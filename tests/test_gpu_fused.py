@@ -140,6 +140,38 @@ def test_fused_backward_equals_op_by_op_bit_for_bit(device, dt, expr, shapes):
     fused.close()
 
 
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("expr,shapes", [
+    ("silu(i0*i1+i1)", [[5, 1, 33], [1, 9, 33]]),            # odd rows; one more position than the steps fetched ahead
+    ("tanh(i0*i1+i1)", [[3, 1, 77], [1, 8, 77]]),            # tanh's rare inputs are looked for in the flat form too
+    ("i0*i1 - i2", [[6, 1, 31], [1, 3, 31], [6, 3, 1]]),     # fewer positions than the steps fetched ahead
+    ("i0*i1+i1", [[2, 3, 1, 35], [1, 1, 7, 35]]),            # two dims summed for i1
+])
+def test_fused_at_odd_extents(device, dt, expr, shapes):
+    """Rows that 128-bit accesses do not fit: the flat forward form and the one-element-per-lane backward form give the bits of the
+    op-by-op evaluation (the gradients because every sum here runs over one node's terms in the same order)."""
+    rng = np.random.default_rng(61)
+    hosts = [rng.uniform(-2.0, 2.0, size=int(np.prod(s))).astype(dt) for s in shapes]
+    hosts[0][:2] = 0, 1e-12
+    out_shape = [max(s[k] for s in shapes) for k in range(len(shapes[0]))]
+    err_h = rng.uniform(-1.0, 1.0, size=int(np.prod(out_shape))).astype(dt)
+
+    def run(make_result):
+        ts = [Tensor.of(dt, s, h).set_rqs_gradient(True).to(device) for s, h in zip(shapes, hosts)]
+        y = make_result(ts)
+        y.backward(Tensor.of(dt, out_shape, err_h))
+        return y.items, [t.gradient.items for t in ts]
+
+    f = Function.of(expr)
+    fused = device.optimized_operation_of(f, "fused_odd_test")
+    y_ref, g_ref = run(lambda ts: f(*ts))
+    y_fus, g_fus = run(lambda ts: fused(*ts))
+    assert _same_bits(y_fus, y_ref)
+    for j, (a, b) in enumerate(zip(g_fus, g_ref)):
+        assert _same_bits(a, b), (j, np.abs(a - b).max())
+    fused.close()
+
+
 def test_fused_backward_of_a_sum_takes_one_kernel_per_input(device, oracle):
     """sum(tanh(a*b+b)).backward() with a [n,1,k], b [1,m,k] through the fused operation: the virtual all-ones error stays
     one element, each gradient is one launch of the gradient kernel, and no result-sized tensor besides the forward
