@@ -412,3 +412,25 @@ def test_argument_errors_are_reported_not_faulted(device):
         gpu_conv(device, np.zeros(16, dtype=dt), ND.of_shape([4, 4]), a, ND.of_shape([4, 4]), b, ND.of_shape([2, 2]))
     with pytest.raises(ValueError, match="rank"):
         gpu_conv(device, np.zeros(1, dtype=dt), ND.of_shape([1] * 9), np.ones(1, dtype=dt), ND.of_shape([1] * 9), np.ones(1, dtype=dt), ND.of_shape([1] * 9))
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("mkn", [(32, 16, 4096), (64, 512, 64), (65, 1023, 71), (200, 333, 177), (40, 5000, 33)])
+@pytest.mark.parametrize("order", ["row", "column"])
+def test_contractions_of_the_multiply_add_family(device, dt, mkn, order):
+    """Tiles of 64 x 64 (F64: FP64 matrix instructions; F32: the small tile), whole and partial, one and several parts along k,
+    operands contiguous along k and along their rows: against a float64 product, and the same bits on every run."""
+    m, k, n = mkn
+    rng = np.random.default_rng(m * 3 + n)
+    a, b = rng.standard_normal(m * k).astype(dt), rng.standard_normal(k * n).astype(dt)
+    ca, cb = ND.of_shape([m, k, 1]), ND.of_shape([1, k, n])
+    A, B = a.reshape(m, k).astype(np.longdouble), b.reshape(k, n).astype(np.longdouble)
+    if order == "column":
+        ca, cb = ND.of_shape([1, k, m]).reshaped([2, 1, 0]), ND.of_shape([n, k, 1]).reshaped([2, 1, 0])
+        A, B = a.reshape(k, m).T.astype(np.longdouble), b.reshape(n, k).T.astype(np.longdouble)
+    runs = [gpu_conv(device, np.zeros(m * n, dtype=dt), ND.of_shape([m, 1, n]), a, ca, b, cb, path=L.NK_CONV_GEMM) for _ in range(2)]
+    assert device.last_conv_path() == L.NK_CONV_GEMM
+    assert np.array_equal(runs[0], runs[1])
+    # rounding of a sum of k products in any order: (k + splits) half units in the last place of sum|a||b|
+    bound = (k + 16) * float(np.finfo(dt).eps) / 2 * (np.abs(A) @ np.abs(B))
+    assert np.all(np.abs(runs[0].reshape(m, n) - A @ B) <= bound)
