@@ -128,3 +128,33 @@ def test_calls_the_family_cannot_take_are_refused_when_forced(device):
     x = np.ones(40 * 16, dtype=F32)
     with pytest.raises(ValueError):      # too small for a 128 x 256 tile to make sense
         gpu_conv(device, np.zeros(40 * 40, dtype=F32), ND.of_shape([40, 1, 40]), x, ND.of_shape([40, 16, 1]), x, ND.of_shape([1, 16, 40]), path=L.NK_CONV_TC)
+
+
+@pytest.mark.parametrize("mkn", [(1999, 70, 2048), (2048, 33, 1921), (2300, 136, 2300)])
+def test_products_on_pairs_of_ctas(device, mkn):
+    """Sizes whose 256 x 256 tiles fill the chip's SM pairs: edges in every direction (the last tile's second CTA partly or wholly
+    outside), one and several accumulation chunks, several tiles per pair. Reference in float64."""
+    m, k, n = mkn
+    rng = np.random.default_rng(m + k)
+    a, b = rng.standard_normal(m * k).astype(F32), rng.standard_normal(k * n).astype(F32)
+    got = gpu_conv(device, np.zeros(m * n, dtype=F32), ND.of_shape([m, 1, n]), a, ND.of_shape([m, k, 1]), b, ND.of_shape([1, k, n]), path=L.NK_CONV_TC)
+    A, B = a.reshape(m, k).astype(np.float64), b.reshape(k, n).astype(np.float64)
+    assert np.all(np.abs(got.reshape(m, n) - A @ B) <= 1e-5 * (np.abs(A) @ np.abs(B)))
+
+
+@pytest.mark.parametrize("mkn", [(64, 512, 64), (130, 4001, 129), (300, 1037, 200), (64, 9000, 500)])
+@pytest.mark.parametrize("order", ["row", "column"])
+def test_products_split_along_k(device, mkn, order):
+    """Few tiles and a long sum: k is split over several CTAs per tile and the parts are added in order -- the same bits on every
+    run -- from operands that are contiguous along k and along their rows, at extents 16-byte loads fit and do not fit."""
+    m, k, n = mkn
+    rng = np.random.default_rng(m + k)
+    a, b = rng.standard_normal(m * k).astype(F32), rng.standard_normal(k * n).astype(F32)
+    ca, cb = ND.of_shape([m, k, 1]), ND.of_shape([1, k, n])
+    A, B = a.reshape(m, k).astype(np.float64), b.reshape(k, n).astype(np.float64)
+    if order == "column":
+        ca, cb = ND.of_shape([1, k, m]).reshaped([2, 1, 0]), ND.of_shape([n, k, 1]).reshaped([2, 1, 0])
+        A, B = a.reshape(k, m).T.astype(np.float64), b.reshape(n, k).T.astype(np.float64)
+    runs = [gpu_conv(device, np.zeros(m * n, dtype=F32), ND.of_shape([m, 1, n]), a, ca, b, cb, path=L.NK_CONV_TC) for _ in range(2)]
+    assert np.array_equal(runs[0], runs[1])
+    assert np.all(np.abs(runs[0].reshape(m, n) - A @ B) <= 1e-5 * (np.abs(A) @ np.abs(B)))
