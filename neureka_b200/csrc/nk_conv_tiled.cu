@@ -113,22 +113,36 @@ static bool nk_describe_for_tma(const nk_buf* buf, const NkView& v, size_t es, b
 // fallback to the gather family that measured 20 times slower. The block comes from the device's stream-ordered pool:
 // copy, kernel and release all queue on the context's stream.
 struct StageDims {
-    int rank;
-    long long total, base;
-    long long div[NK_MAX_RANK], sstride[NK_MAX_RANK], dstride[NK_MAX_RANK];
+    int n_outer;                                   // dims before the last
+    long long rows, base;
+    int width;                                     // extent of the last dim
+    long long sx;                                  // its source stride
+    long long ext[NK_MAX_RANK], sstride[NK_MAX_RANK];
+    long long pitch;                               // elements per copied row
 };
+// A row per warp and step: one decode of the row index, then coalesced runs, four loads per lane in flight.
+// 16x16x131x127 F32: 13 us; decoding every element with 64-bit divisions: 41.
 template <class T>
-__global__ void __launch_bounds__(256) nk_stage_kernel(T* __restrict__ dst, const T* __restrict__ src, StageDims d) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < d.total; i += stride) {
-        long long rem = i, so = d.base, dof = 0;
-        for (int k = 0; k < d.rank; k++) {
-            const long long idx = rem / d.div[k];
-            rem -= idx * d.div[k];
-            so += idx * d.sstride[k];
-            dof += idx * d.dstride[k];
+__global__ void __launch_bounds__(256) nk_stage_kernel(T* __restrict__ dst, const T* __restrict__ src, const StageDims d) {
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * 8;
+    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < d.rows; r += warps) {
+        long long rem = r, so = d.base;
+        for (int k = d.n_outer - 1; k >= 0; k--) {
+            const long long q = rem / d.ext[k];
+            so += (rem - q * d.ext[k]) * d.sstride[k];
+            rem = q;
         }
-        dst[dof] = src[so];
+        T* out = dst + r * d.pitch;
+        for (int x = lane; x < d.width; x += 128) {
+            T v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (x + 32 * u < d.width) v[u] = src[so + (x + 32 * u) * d.sx];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (x + 32 * u < d.width) out[x + 32 * u] = v[u];
+        }
     }
 }
 struct Staged {
@@ -143,20 +157,22 @@ static int nk_stage_operand(nk_ctx* ctx, int dtype, const nk_buf* src, const NkV
     const int64_t pitch = ((v.shape[X] + cw - 1) / cw) * cw;
     StageDims d;
     memset(&d, 0, sizeof(d));
-    d.rank = rank;
+    d.n_outer = rank - 1;
     d.base = v.base;
+    d.width = int(v.shape[X]);
+    d.sx = v.estride[X];
+    d.pitch = pitch;
     out->view = v;
     out->view.base = 0;
-    int64_t ds = 1, dv = 1;
+    d.rows = 1;
+    int64_t ds = 1;
     for (int k = rank - 1; k >= 0; k--) {
-        d.div[k] = dv;
-        dv *= v.shape[k];
+        d.ext[k] = v.shape[k];
         d.sstride[k] = v.estride[k];
-        d.dstride[k] = ds;
+        if (k != X) d.rows *= v.shape[k];
         out->view.estride[k] = ds;
         ds *= (k == X) ? pitch : v.shape[k];
     }
-    d.total = dv;
     out->view.dense_row_major = pitch == v.shape[X];
     if (ds >= (int64_t(1) << 40)) return -1;
     void* ptr = nullptr;
@@ -167,7 +183,7 @@ static int nk_stage_operand(nk_ctx* ctx, int dtype, const nk_buf* src, const NkV
     out->buf.n_elems = ds;
     out->buf.owned = false;
     out->used = true;
-    const int grid = nk_grid_for(ctx, d.total, 256, 16);
+    const int grid = nk_grid_for(ctx, d.rows, 8, 16);
     if (dtype == NK_F32) nk_stage_kernel<float><<<grid, 256, 0, ctx->stream>>>(static_cast<float*>(ptr), static_cast<const float*>(src->ptr), d);
     else nk_stage_kernel<double><<<grid, 256, 0, ctx->stream>>>(static_cast<double*>(ptr), static_cast<const double*>(src->ptr), d);
     return nk_after_launch(ctx, "nk_stage_kernel");

@@ -271,13 +271,10 @@ int nk_launch_wgrad(nk_ctx* ctx, T* out, WgradPlan& p, const TmaImage& imgA, con
     p.tilesX = (p.EW + C::TW - 1) / C::TW;
     p.tilesY = p.has_y ? (p.EH + C::TH - 1) / C::TH : 1;
     p.units = p.NQ * int64_t(p.tilesY) * p.tilesX;
-    cudaError_t e = cudaFuncSetAttribute(nk_conv_wgrad_kernel<T, KH, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) return nk_cuda_fail(ctx, e, "cudaFuncSetAttribute(nk_conv_wgrad_kernel)");
     // as many CTAs as are resident at once (KH*KW accumulators per thread decide that), so that the grid is one wave
     int per_sm = 1;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nk_conv_wgrad_kernel<T, KH, KW>, 288, smem);
-    if (e != cudaSuccess) return nk_cuda_fail(ctx, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(nk_conv_wgrad_kernel)");
-    if (per_sm < 1) per_sm = 1;
+    const int ost = nk_tiled_occupancy(ctx, reinterpret_cast<const void*>(nk_conv_wgrad_kernel<T, KH, KW>), 288, smem, &per_sm);
+    if (ost) return ost;
     int64_t chunks = int64_t(ctx->prop.multiProcessorCount) * per_sm / p.NP;
     if (chunks > p.units) chunks = p.units;
     if (chunks > 4096) chunks = 4096;
