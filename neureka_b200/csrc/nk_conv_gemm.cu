@@ -197,6 +197,10 @@ struct DgemmSplit {
 __device__ __forceinline__ void dg_mma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
+// TABLES: some index group goes through an offset table. Otherwise an element's address is one base per operand and thread plus
+// a constant step, moved on by a panel at a time: with the offsets worked out per element, the integer chains took longer than
+// the products (777 x 1023 x 515: 59 us, with offsets per element 79; 128 x 64 tiles of multiply-adds: 172).
+template <bool TABLES>
 __global__ void __launch_bounds__(128, 3) nk_conv_dgemm_kernel(double* __restrict__ out, const double* __restrict__ A, const double* __restrict__ B,
                                                                const GemmView p, const DgemmSplit sp) {
     __shared__ double As[2][DG_T][DG_PITCH], Bs[2][DG_T][DG_PITCH];
@@ -214,20 +218,47 @@ __global__ void __launch_bounds__(128, 3) nk_conv_dgemm_kernel(double* __restric
         else { *r = tid & 63; *k = (tid >> 6) + 2 * i; }
     };
     double ra[8], rb[8];
-    auto fetch = [&](int64_t k0) {   // rows past the edge are clamped (their products are never stored), the k tail is zero
+    // rows past the edge and the k tail read as zero
+    struct Walk { const double* at; int64_t step, panel; unsigned rows; int k; };   // rows: bit i = element i's row exists
+    auto walk = [&](const double* base, const GemmOff& R, const GemmOff& K, int64_t row0, int64_t n_rows, int kfast) {
+        Walk w;
+        int r0, r;
+        place(kfast, 0, &r0, &w.k);
+        w.at = base + (row0 + r0) * R.stride + (k_begin + w.k) * K.stride;
+        w.step = kfast ? 8 * R.stride : 2 * K.stride;
+        w.panel = DG_K * K.stride;
+        w.rows = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            int r, k;
-            place(sp.a_kfast, i, &r, &k);
-            const int64_t m = m0 + r < p.M ? m0 + r : p.M - 1;
-            ra[i] = k0 + k < k_end ? A[p.bA + p.Am.at(m) + p.Ak.at(k0 + k)] : 0.0;
+            int k;
+            place(kfast, i, &r, &k);
+            if (row0 + r < n_rows) w.rows |= 1u << i;
         }
+        return w;
+    };
+    Walk wa = walk(A + p.bA, p.Am, p.Ak, m0, p.M, sp.a_kfast), wb = walk(B + p.bB, p.Bn, p.Bk, n0, p.N, sp.b_kfast);
+    auto pull = [&](Walk& w, int kfast, int left, double (&v)[8]) {   // left: k of the panel that exist
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            int r, k;
-            place(sp.b_kfast, i, &r, &k);
-            const int64_t n = n0 + r < p.N ? n0 + r : p.N - 1;
-            rb[i] = k0 + k < k_end ? B[p.bB + p.Bn.at(n) + p.Bk.at(k0 + k)] : 0.0;
+            const int k = kfast ? w.k : w.k + 2 * i;
+            v[i] = ((w.rows >> i) & 1u) && k < left ? w.at[i * w.step] : 0.0;
+        }
+        w.at += w.panel;
+    };
+    auto fetch = [&](int64_t k0) {
+        if constexpr (!TABLES) {
+            const int left = k_end - k0 < DG_K ? int(k_end - k0) : DG_K;
+            pull(wa, sp.a_kfast, left, ra);
+            pull(wb, sp.b_kfast, left, rb);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                int r, k;
+                place(sp.a_kfast, i, &r, &k);
+                ra[i] = m0 + r < p.M && k0 + k < k_end ? A[p.bA + p.Am.at(m0 + r) + p.Ak.at(k0 + k)] : 0.0;
+                place(sp.b_kfast, i, &r, &k);
+                rb[i] = n0 + r < p.N && k0 + k < k_end ? B[p.bB + p.Bn.at(n0 + r) + p.Bk.at(k0 + k)] : 0.0;
+            }
         }
     };
     auto stash = [&](int buf) {
@@ -380,7 +411,8 @@ int launch_gemm(nk_ctx* ctx, double* out, const double* A, const double* B, cons
         sp.tickets = reinterpret_cast<int*>(static_cast<char*>(rest) + part_bytes);
         NK_CUDA(ctx, cudaMemsetAsync(sp.tickets, 0, ticket_bytes, ctx->stream));
     }
-    nk_conv_dgemm_kernel<<<unsigned(tiles * sp.splits), 128, 0, ctx->stream>>>(out, A, B, gemm_view(p, tab), sp);
+    if (tab) nk_conv_dgemm_kernel<true><<<unsigned(tiles * sp.splits), 128, 0, ctx->stream>>>(out, A, B, gemm_view(p, tab), sp);
+    else nk_conv_dgemm_kernel<false><<<unsigned(tiles * sp.splits), 128, 0, ctx->stream>>>(out, A, B, gemm_view(p, tab), sp);
     return nk_after_launch(ctx, "nk_conv_gemm_kernel");
 }
 

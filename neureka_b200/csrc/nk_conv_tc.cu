@@ -24,7 +24,8 @@
 // Two shapes of step 3, chosen by estimated time (see nk_conv_tc_try):
 //   * pairs of CTAs (cta_group::2), tile 256 x 256: each CTA stages 128 rows of A and 128 of B, 32 KiB per 16 k where a lone
 //     CTA with a 128 x 256 tile stages 48. Six products of 128 x 256 x 8 take 768 cycles; the lone CTA moved 48 KiB in and
-//     72 KiB out of its shared memory per stage in that time, more than the 128 bytes per cycle there are, the pair 32 + 48;
+//     72 KiB out of its shared memory per stage in that time, more than the 128 bytes per cycle there are, the pair 32 + 48.
+//     4096^3: 554 us, lone CTAs 596;
 //   * lone CTAs, tile 128 x 128, for products with too few large tiles to fill the chip; where even these are too few, k is
 //     split over several CTAs per tile: each warp leaves its part of the tile in scratch and takes a ticket, the warp that
 //     draws the last one adds the parts in split order (nobody waits; the result does not depend on the order of arrival).
@@ -102,7 +103,7 @@ struct TcSplit {
 // direction (rows x k, or -- turned through shared memory on the way -- k x rows), four 16-byte loads per thread in flight
 // and 16-byte stores; operands that 16-byte loads do not fit are read element by element. Both operands in one launch: the
 // second's tiles follow the first's. Bound by memory: 12 bytes move per element.
-// 4096^2 operands, two per product: 116 us with 4-byte accesses and 32 x 32 tiles, 58 us is the floor.
+// 4096^2 operands, two per product: 62 us (58 is the floor); two launches of 32 x 32 tiles with 4-byte accesses: 87 to 114.
 __global__ void __launch_bounds__(256) nk_tc_split_kernel(const TcSplit p) {
     __shared__ float tile[32][129];
     const int which = int64_t(blockIdx.x) >= p.op[0].tiles ? 1 : 0;
