@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) nk_fill_fun_kernel(T* __restrict__ out, E
 // The 128 elements of a tile are added in index order by one lane, so the work is turned through shared memory:
 //   * nk_sum_rows_kernel (contiguous, 16-byte aligned): a warp requests 32 whole tiles with 16-byte asynchronous copies, into rows
 //     padded by 16 bytes, and lane t then adds row t. The copies need no registers: twelve warps' 16 KB each are in flight per
-//     SM. 2^26 F32 elements: 48 us (40 is the floor); sixteen elements of a tile at a time through registers: 170 us.
+//     SM. 2^26 F32 elements: 46 us (40 is the floor); one tile per warp, one lane adding: 487.
 //   * nk_sum_tiles_kernel (any view): the same through registers, 16 elements of every tile at a time.
 //   * nk_sum_last_kernel: at most 128 tiles, i.e. the last two levels of any sum (or all of a sum of up to 2^14 elements) in
 //     one CTA: a warp stages a tile, one lane adds it; one lane then adds the tile sums.
