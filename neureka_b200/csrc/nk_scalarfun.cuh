@@ -126,6 +126,12 @@ __device__ __forceinline__ float sig32(float x) {
     const float y = float(sig_lean(double(fminf(fmaxf(x, -700.0f), 700.0f))));
     return x != x ? x + x : y;
 }
+// gelu's sigmoid as its derivative uses it, rounded to F32 by itself. This and sig32 give the bits of float(sig64(..)) for all
+// 2^32 inputs (swept), so the derivatives below lost nothing with the library's exp and division.
+__device__ __forceinline__ float gelu_sig32(float x) {
+    const float y = float(sig_lean(double(fminf(fmaxf(x, -411.0f), 411.0f)) * 1.702));
+    return x != x ? x + x : y;
+}
 __device__ __forceinline__ float silu32(float x) {
     const float y = float(double(x) * sig_lean(double(fminf(fmaxf(x, -700.0f), 700.0f))));
     return (x != x || x == __int_as_float(0xff800000)) ? x - x : y;
@@ -236,7 +242,7 @@ __device__ __forceinline__ float fun(int f, bool derive, float x) {
             return -temp * tanh2 + temp;
         }
         case NK_FUN_FAST_GAUS: { float x2 = x * x; return -2 * x / (x2 * x2 + 2 * x2 + 1); }
-        case NK_FUN_GELU: { float s = float(sig64(double(x) * 1.702)); float ds = s * (1.0f - s); return s + ds * x * 1.702f; }
+        case NK_FUN_GELU: { float s = gelu_sig32(x); float ds = s * (1.0f - s); return s + ds * x * 1.702f; }
         case NK_FUN_IDY: return 1;
         case NK_FUN_LOG10: return 1 / (x * float(log(10.0)));
         case NK_FUN_LN: return 1.0f / x;
@@ -246,8 +252,8 @@ __device__ __forceinline__ float fun(int f, bool derive, float x) {
             if (x > 0) return float(NKF_SELU_SCALE);
             else if (x <= 0) return float(NKF_SELU_SCALE * NKF_SELU_ALPHA * exp(double(x)));
             else return __int_as_float(0x7fc00000);
-        case NK_FUN_SILU: { float s = float(sig64(double(x))); return s + (x * s * (1.0f - s)); }
-        case NK_FUN_SIG: { float s = float(sig64(double(x))); return s * (1 - s); }
+        case NK_FUN_SILU: { float s = sig32(x); return s + (x * s * (1.0f - s)); }
+        case NK_FUN_SIG: { float s = sig32(x); return s * (1 - s); }
         case NK_FUN_SOFTSIGN: return 1.0f / (2.0f * fabsf(x) + x * x + 1.0f);
         case NK_FUN_SQRT: return 0.5f * inv_sqrt(x);
         case NK_FUN_TANH: { double t = double(tanh32(x)); return float(1 - t * t); }
