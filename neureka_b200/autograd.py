@@ -222,9 +222,15 @@ def evaluate(node, inputs: List[Tensor], do_ad: bool) -> Tensor:
     return acc
 
 
-def _accumulate(t: Tensor, err: Tensor) -> None:
-    """TensorImpl.addToGradient (:1275-1300): first error becomes the gradient, later ones are added in place."""
+def _accumulate(t: Tensor, err: Tensor, owned: bool = False) -> None:
+    """TensorImpl.addToGradient (:1275-1300): first error becomes the gradient, later ones are added in place. An error that
+    nobody else holds (`owned`) becomes the gradient itself; any other is copied -- a launch and a pass over the tensor that
+    a training step pays per parameter."""
     if t.gradient is None:
+        if owned and err.shape == t.shape and err.dtype == t.dtype and not err.is_virtual and not err.is_slice() and err.ndconf.is_simple():
+            err.is_intermediate = False
+            t.gradient = err
+            return
         g = err.device.new_tensor(t.dtype, t.shape)
         if err.shape != t.shape:
             err = _view_as(err, t.shape)
@@ -278,16 +284,19 @@ def backward(result: Tensor, error: Optional[Tensor] = None) -> None:
             order.append(t)
             stack.pop()
     pending = {id(result): error}
+    shared = {id(error)}   # errors that the caller or another node holds too: never handed out as a gradient
     for t in reversed(order):
         err = pending.pop(id(t), None)
         if err is None:
             continue
         if t.rqs_gradient:
-            _accumulate(t, err)
+            _accumulate(t, err, id(err) not in shared)
         if t.graph_node is None:
             continue
         for p, act in t.graph_node.parents:
             e = act(err)
+            if e is err:
+                shared.add(id(err))
             if id(p) in pending:
                 pending[id(p)] = F.run_operator("+", pending[id(p)], e)
             else:

@@ -309,3 +309,27 @@ def test_results_of_a_step_are_released_with_their_last_reference(device):
         assert device.number_of_data_objects() == n0 and device.number_of_stored() == t0
     finally:
         gc.enable()
+
+
+def test_gradients_are_tensors_of_their_own(device):
+    """An error becomes a gradient without a copy only where nobody else holds it: not the caller's, and not one that a sum passes
+    on to two tensors. Adding to one gradient in a second backward pass leaves the others and the caller's error alone."""
+    rng = np.random.default_rng(3)
+    x, y = (Tensor.of(np.float32, [4, 35], rng.standard_normal(140).astype(np.float32)).set_rqs_gradient(True).to(device) for _ in range(2))
+    z = Tensor.of(np.float32, [1, 35], rng.standard_normal(35).astype(np.float32)).set_rqs_gradient(True).to(device)
+    e_h = rng.standard_normal(140).astype(np.float32)
+    e = Tensor.of(np.float32, [4, 35], e_h).to(device)
+    f = Function.of("(i0 + i2) * i1")
+    out = f(x, y, z)
+    out.backward(e)
+    g = (e_h.reshape(4, 35) * y.numpy()).astype(np.float32)
+    assert np.array_equal(x.gradient.numpy(), g)
+    assert len({id(t._data) for t in (x.gradient, y.gradient, z.gradient, e)}) == 4
+    gz, gy = z.gradient.numpy().copy(), y.gradient.numpy().copy()
+    (x + z).backward(e)
+    assert np.array_equal(x.gradient.numpy(), g + e_h.reshape(4, 35))
+    assert np.array_equal(y.gradient.numpy(), gy) and not np.array_equal(z.gradient.numpy(), gz)
+    assert np.array_equal(e.numpy().reshape(-1), e_h)
+    w = Tensor.of(np.float32, [4, 35], e_h).set_rqs_gradient(True).to(device)
+    (w + z).backward(e)   # the caller's error reaches w unchanged: copied
+    assert w.gradient._data is not e._data and np.array_equal(w.gradient.numpy(), e.numpy())
