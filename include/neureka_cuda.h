@@ -143,6 +143,10 @@ int nk_binary(nk_ctx* ctx, int32_t op, int32_t dtype, int32_t rank,
 int nk_unary(nk_ctx* ctx, int32_t fun, int32_t dtype, int32_t rank,
              nk_buf* drn, const int32_t* cfg0, nk_buf* src, const int32_t* cfg1, int32_t d);
 
+/* drain = f(src) and ddrain = f'(src) in one pass over src: what nk_unary gives with d < 0 and d >= 0, bit for bit. */
+int nk_unary_both(nk_ctx* ctx, int32_t fun, int32_t dtype, int32_t rank,
+                  nk_buf* drn, const int32_t* cfg0, nk_buf* ddrn, const int32_t* cfgd, nk_buf* src, const int32_t* cfg1);
+
 /* Algorithm BiScalarBroadcast: replaces CLScalarBroadcast* (J/backend/main/implementations/broadcast/CLScalarBroadcast.java:16-64 +
  * kernels/scalarization_template.cl), semantics of CPUScalarBroadcast.java:29-75: drn = f(src, value). */
 int nk_scalar_binary(nk_ctx* ctx, int32_t op, int32_t dtype, int32_t rank,

@@ -86,6 +86,7 @@ SIGNATURES = {
     "nk_broadcast": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _cfg, _vp, _cfg, _vp, _cfg, _i32]),
     "nk_binary": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _cfg, _vp, _cfg, _vp, _cfg, _i32]),
     "nk_unary": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _cfg, _vp, _cfg, _i32]),
+    "nk_unary_both": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _cfg, _vp, _cfg, _vp, _cfg]),
     "nk_scalar_binary": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _cfg, _vp, _cfg, _dbl, _i32]),
     "nk_fill_fun": (C.c_int, [_vp, _i32, _i32, _i32, _vp, _cfg, _dbl, _i32]),
     "nk_sum": (C.c_int, [_vp, _i32, _i32, _vp, _cfg, _vp, _i64]),

@@ -137,9 +137,7 @@ def _reshape_like(g: Tensor, like: Tensor) -> Tensor:
     return g
 
 
-def _record_function(fid: str, x: Tensor, out: Tensor) -> None:
-    if not _tracks(x):
-        return
+def _record_function(fid: str, x: Tensor, out: Tensor, deriv: Optional[Tensor]) -> None:
     if fid == "sumItems":
         def action(err, x=x):
             dev = err.device
@@ -149,8 +147,7 @@ def _record_function(fid: str, x: Tensor, out: Tensor) -> None:
             return full
         out.graph_node = GraphNode(out, [(x, action)])
         return
-    deriv = F.run_function(fid, x, 0)   # eager local derivative (FallbackAlgorithm.java:118-129)
-    deriv.is_intermediate = False
+    deriv.is_intermediate = False   # eager local derivative (FallbackAlgorithm.java:118-129)
 
     def action(err, deriv=deriv):
         return _mul(err, deriv)
@@ -192,9 +189,13 @@ def evaluate(node, inputs: List[Tensor], do_ad: bool) -> Tensor:
         return Tensor.of(like.dtype, (1,), [node.value])
     if node.kind == "fun":
         x = evaluate(node.children[0], inputs, do_ad)
-        out = F.run_function(node.value, x)
-        if do_ad:
-            _record_function(node.value, x, out)
+        if not (do_ad and _tracks(x)):
+            return F.run_function(node.value, x)
+        if node.value == "sumItems":
+            out, deriv = F.run_function(node.value, x), None
+        else:
+            out, deriv = F.run_function_and_derivative(node.value, x)
+        _record_function(node.value, x, out, deriv)
         return out
     sym = node.value
     vals = [evaluate(c, inputs, do_ad) for c in node.children]

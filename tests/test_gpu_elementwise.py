@@ -311,3 +311,23 @@ def test_transposed_operands_and_odd_rows(device, dt, shape):
     cr = ND.of_shape([1] * (rank - 1) + [shape[-1]])
     got = gpu_call3(L.lib.nk_broadcast, device, L.OPS["-"], np.zeros(dense.size, dtype=dt), dense, a, dense, row, cr)
     assert np.array_equal(got.reshape(shape), av - row)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("fun", L.FUN_IDS)
+def test_value_and_derivative_in_one_pass(device, dt, fun):
+    """nk_unary_both against nk_unary twice, bit for bit: dense tensors (vector tail included), an unaligned start and a strided
+    source (two launches), with the inputs tanh repairs among them."""
+    rng = np.random.default_rng(67)
+    n = 1027
+    x = _inputs(rng, 2 * n + 1, dt, fun)
+    x[:6] = np.asarray([0.0, 1e-12, -1e-9, 30.0, -30.0, np.inf], dtype=dt) if fun not in ("ln", "log10", "sqrt", "cbrt") else x[:6]
+    dense, parent = ND.of_shape([n]), ND.of_shape([2 * n + 1])
+    k0, p0 = cfgp(dense)
+    S, D, E = DevArray(device, x), DevArray(device, np.zeros(n, dtype=dt)), DevArray(device, np.zeros(n, dtype=dt))
+    for conf in (parent.sliced([n], [0], [1]), parent.sliced([n], [1], [1]), parent.sliced([n], [1], [2])):
+        k1, p1 = cfgp(conf)
+        L.check(L.lib.nk_unary_both(device.ctx, L.FUN[fun], S.nk_dtype, 1, D.buf, p0, E.buf, p0, S.buf, p1), device.ctx)
+        for got, d in ((D.read(), -1), (E.read(), 0)):
+            assert np.array_equal(got, gpu_unary(device, L.FUN[fun], np.zeros(n, dtype=dt), dense, x, conf, d=d), equal_nan=True), (fun, d)
+    assert L.lib.nk_unary_both(device.ctx, 99, S.nk_dtype, 1, D.buf, p0, E.buf, p0, S.buf, p0) == L.NK_ERR_BAD_ARG
