@@ -13,6 +13,7 @@
 //
 // F32: plain FMAs (the large F32 products go to nk_conv_tc.cu). F64: nk_conv_dgemm_kernel below, FP64 matrix instructions.
 #include "nk_gemm_plan.h"
+#include "nk_launch_rules.h"
 
 namespace {
 
@@ -185,9 +186,10 @@ __global__ void __launch_bounds__(256, 2) nk_conv_gemm_kernel(T* __restrict__ ou
 // on every eight. A CTA of four warps takes a 64 x 64 tile, a warp 32 x 32 of it (16 blocks, 64 accumulator registers); panels of
 // 16 k lie k fastest in shared memory with a pitch of 20 doubles, which puts the 4 x 4 (row, k) elements of a half warp's
 // fragment load on 16 different banks. The next panel travels through registers while this one is multiplied.
-// Where the tiles are too few or fill the last wave badly, k is split over several CTAs per tile; every warp leaves its part in
+// Where the tiles are few or fill the last wave badly, k is split over several CTAs per tile (nk_dgemm_parts); every warp leaves its part in
 // scratch and draws a ticket, and the one with the last ticket adds the parts in split order (nobody waits, same bits always).
-constexpr int DG_T = 64, DG_K = 16, DG_PITCH = 20, DG_MAX_SPLITS = 16;
+constexpr int DG_T = 64, DG_K = 16, DG_PITCH = 20;
+static_assert(DG_T * DG_T * sizeof(double) == NK_DGEMM_PART_BYTES, "a part is one tile of sums");
 struct DgemmSplit {
     int splits, kb_per;           // k blocks of DG_K per part
     double* parts;                // [tile][part][warp of 4][16 blocks][32 lanes x 2]
@@ -384,32 +386,28 @@ int launch_gemm(nk_ctx* ctx, double* out, const double* A, const double* B, cons
     const int64_t sms = ctx->prop.multiProcessorCount;
     const int64_t tiles = ((p.M + DG_T - 1) / DG_T) * ((p.N + DG_T - 1) / DG_T);
     if (tiles > 0x3ffffffLL) return -1;
-    // k split: the number of parts with the least estimated time -- the FP64 pipes of an SM are shared by its CTAs, so the time is
-    // that of the SM with the most k blocks (1024 cycles each), plus the parts' way through L2
     const int64_t kb = (p.K + DG_K - 1) / DG_K;
-    int64_t best = -1;
-    int splits = 1;
-    for (int s = 1; s <= DG_MAX_SPLITS && s <= kb / 4; s++) {
-        const int64_t per = (kb + s - 1) / s;
-        const int64_t est = ((tiles * s + sms - 1) / sms) * per * 1024 + (s > 1 ? 4000 + 600 * s : 0);
-        if (best < 0 || est < best) { best = est; splits = s; }
-    }
+    NkDgemmParts parts = nk_dgemm_parts(tiles, kb, sms);
     DgemmSplit sp;
     memset(&sp, 0, sizeof(sp));
-    sp.kb_per = int((kb + splits - 1) / splits);
-    sp.splits = int((kb + sp.kb_per - 1) / sp.kb_per);
     sp.a_kfast = p.k.n > 0 && p.k.sa[p.k.n - 1] == 1;
     sp.b_kfast = p.k.n > 0 && p.k.sb[p.k.n - 1] == 1;
-    const size_t part_bytes = sp.splits > 1 ? size_t(tiles) * sp.splits * DG_T * DG_T * sizeof(double) : 0;
-    const size_t ticket_bytes = sp.splits > 1 ? size_t(tiles) * 4 * sizeof(int) : 0;
     const int64_t* tab;
     void* rest;
-    const int st = gemm_scratch(ctx, p, part_bytes + ticket_bytes, &tab, &rest);
+    auto part_bytes = [&] { return parts.splits > 1 ? size_t(tiles) * parts.splits * NK_DGEMM_PART_BYTES : 0; };
+    auto ticket_bytes = [&] { return parts.splits > 1 ? size_t(tiles) * 4 * sizeof(int) : 0; };
+    int st = gemm_scratch(ctx, p, part_bytes() + ticket_bytes(), &tab, &rest);
+    if (st == NK_ERR_OOM && parts.splits > 1) {   // the parts are only there for speed
+        parts = NkDgemmParts{1, kb};
+        st = gemm_scratch(ctx, p, 0, &tab, &rest);
+    }
     if (st) return st;
+    sp.splits = parts.splits;
+    sp.kb_per = int(parts.kb_per);
     if (sp.splits > 1) {
         sp.parts = static_cast<double*>(rest);
-        sp.tickets = reinterpret_cast<int*>(static_cast<char*>(rest) + part_bytes);
-        NK_CUDA(ctx, cudaMemsetAsync(sp.tickets, 0, ticket_bytes, ctx->stream));
+        sp.tickets = reinterpret_cast<int*>(static_cast<char*>(rest) + part_bytes());
+        NK_CUDA(ctx, cudaMemsetAsync(sp.tickets, 0, ticket_bytes(), ctx->stream));
     }
     if (tab) nk_conv_dgemm_kernel<true><<<unsigned(tiles * sp.splits), 128, 0, ctx->stream>>>(out, A, B, gemm_view(p, tab), sp);
     else nk_conv_dgemm_kernel<false><<<unsigned(tiles * sp.splits), 128, 0, ctx->stream>>>(out, A, B, gemm_view(p, tab), sp);

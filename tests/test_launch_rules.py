@@ -1,0 +1,56 @@
+"""The launch-shape rules of csrc/nk_launch_rules.h, compiled for the host (no GPU needed)."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+HEADER = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "neureka_b200", "csrc", "nk_launch_rules.h")
+SOURCE = """
+#include "%s"
+extern "C" void dgemm_parts(int64_t tiles, int64_t k_panels, int64_t sms, int64_t* out) {
+    const NkDgemmParts p = nk_dgemm_parts(tiles, k_panels, sms);
+    out[0] = p.splits;
+    out[1] = p.kb_per;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    src, lib = d / "rules.cpp", d / "librules.so"
+    src.write_text(SOURCE % HEADER)
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-fPIC", "-shared", "-o", str(lib), str(src)], check=True)
+    return C.CDLL(str(lib))
+
+
+def dgemm_parts(rules, m, k, n, sms=148):
+    out = (C.c_int64 * 2)()
+    tiles = -(-m // 64) * -(-n // 64)
+    rules.dgemm_parts(C.c_int64(tiles), C.c_int64(-(-k // 16)), C.c_int64(sms), out)
+    return tiles, int(out[0]), int(out[1])
+
+
+@pytest.mark.parametrize("mkn", [(4096, 4096, 4096), (6000, 6000, 6000), (8192, 8192, 8192), (16384, 16384, 16384), (16384, 4096, 16384),
+                                 (40000, 2048, 40000), (49152, 2048, 49152), (3000, 100000, 3000)])
+def test_large_f64_products_need_no_scratch_for_parts(rules, mkn):
+    """Products with many tiles fill the chip by themselves: splitting k would write and read back 64 KB per part."""
+    tiles, splits, kb_per = dgemm_parts(rules, *mkn)
+    assert splits == 1 and kb_per * 16 >= mkn[1]
+
+
+def test_parts_of_f64_products_are_bounded_and_cover_k(rules):
+    for m in (64, 200, 777, 1536, 2048, 3000, 10000, 50000):
+        for n in (64, 515, 1280, 2048, 9000):
+            for k in (16, 100, 1023, 4096, 20000, 1 << 20, (1 << 33) + 5):
+                for sms in (1, 132, 148):
+                    tiles, splits, kb_per = dgemm_parts(rules, m, k, n, sms)
+                    panels = -(-k // 16)
+                    assert 1 <= splits <= 16 and (splits - 1) * kb_per < panels <= splits * kb_per    # every part has work
+                    assert splits == 1 or tiles * splits * 32768 <= 64 << 20
+
+
+def test_few_tiles_and_a_long_sum_are_split(rules):
+    assert dgemm_parts(rules, 64, 20000, 64)[1] == 16
+    assert dgemm_parts(rules, 777, 1023, 515)[1] > 1
