@@ -13,6 +13,7 @@
 // NVRTC is looked up with dlopen at the first compilation (no link-time dependency); the compiled image is loaded
 // with the runtime's library API. A failure to find or run the compiler is reported, nothing falls back.
 #include "nk_internal.h"
+#include "nk_launch_rules.h"
 
 #include <dlfcn.h>
 
@@ -79,9 +80,10 @@ struct FusedGrad {
 
 struct nk_fused {
     cudaLibrary_t lib = nullptr;
-    cudaKernel_t kernel = nullptr;        // forward: flat form; backward: the gradient kernel
+    cudaKernel_t kernel = nullptr;        // forward: flat form; backward: one element and one position at a time
     cudaKernel_t rows1 = nullptr, rows2 = nullptr;   // forward, rows form with one / two outer dims
     cudaKernel_t flat32 = nullptr;                   // forward, flat form of up to 2^31 elements in three merged dims
+    cudaKernel_t grad_vec = nullptr, grad_steps = nullptr;   // backward: a vector per thread / several positions at a time
     int grad_target = -1;                 // >= 0: a backward operation for this input
     int n_leaves = 0;
     int dtype = NK_F32;
@@ -388,11 +390,10 @@ struct FusedGrad {
 };
 __device__ __forceinline__ void nk_terms(T e, T x0, T x1, T x2, T x3, T x4, T x5, T* term) { NK_TERMS }
 
-// Two forms. VEC = a 128-bit vector of target elements per thread and one position at a time: nothing (or next to nothing)
-// is summed. STEPS > 1: one element per thread, the lowest reduced dim walked STEPS positions at a time with all their
-// operands requested before the first (ordered) addition -- a target has few elements, so few threads have to keep the memory
-// system busy, and neighbouring lanes still read neighbouring elements. Gradients of silu(a*b+b), 100 x 333 x 777 F32: 130 and
-// 108 us; a position at a time: 218 and 146.
+// VEC: target elements per thread (a 128-bit vector, or one). STEPS: positions of the lowest reduced dim whose operands are
+// requested together, before the first of their (ordered) additions -- a target of few elements has few threads to keep the memory
+// system busy. Of what is left of the dim, more than half a group is evaluated as a group whose positions past the end are not
+// added (the arithmetic of a group overlaps: eight positions cost about as much as five by themselves), less goes one by one.
 template <int VEC, int STEPS>
 __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
     T* out = reinterpret_cast<T*>(a.out);
@@ -433,7 +434,6 @@ __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
         for (int j = 0; j < NK_NIN; j++) i0[j] = a.nr > 0 ? a.rs[j][0] : 0;
         long long q[NK_MAX_RANK];
         for (int k = 0; k < a.nr; k++) q[k] = 0;
-        // (positions past the end are evaluated and not added: a branch per step would keep the steps' arithmetic from overlapping)
         auto step = [&](const T (*xs)[VEC], bool add) {
 #pragma unroll
             for (int e = 0; e < VEC; e++) {
@@ -464,13 +464,28 @@ __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
                 }
             }
         };
-        while (true) {
-            for (long long r = 0; r < n0; r += STEPS) {
+        if (STEPS == 1 && a.nr == 0) step(x, true);   // nothing is summed: every operand has been read
+        else while (true) {
+            long long r = 0;
+            for (; r + STEPS <= n0; r += STEPS) {
+                T xs[STEPS][NK_NIN + 1][VEC];
+#pragma unroll
+                for (int u = 0; u < STEPS; u++) load(xs[u], r + u);
+#pragma unroll
+                for (int u = 0; u < STEPS; u++) step(xs[u], true);
+            }
+            if (STEPS > 1 && n0 - r > STEPS / 2) {
                 T xs[STEPS][NK_NIN + 1][VEC];
 #pragma unroll
                 for (int u = 0; u < STEPS; u++) load(xs[u], r + u < n0 ? r + u : n0 - 1);
 #pragma unroll
                 for (int u = 0; u < STEPS; u++) step(xs[u], r + u < n0);
+                r = n0;
+            }
+            for (; STEPS > 1 && r < n0; r++) {
+                T xs[1][NK_NIN + 1][VEC];
+                load(xs[0], r);
+                step(xs[0], true);
             }
             int k = 1;
             for (; k < a.nr; k++) {
@@ -496,9 +511,10 @@ __device__ __forceinline__ void nk_grad_body(const FusedGrad& a) {
         else out[o0] = res[0];
     }
 }
-extern "C" __global__ void __launch_bounds__(256) nk_fused_grad_kernel(const FusedGrad a) {
-    if (a.vec > 1) nk_grad_body<VECW, 1>(a); else nk_grad_body<1, 8>(a);
-}
+// Kernels of their own: in one kernel the vector form had the registers, and the occupancy, of the eight-step form.
+extern "C" __global__ void __launch_bounds__(256) nk_fused_grad_one(const FusedGrad a) { nk_grad_body<1, 1>(a); }
+extern "C" __global__ void __launch_bounds__(256) nk_fused_grad_vec(const FusedGrad a) { nk_grad_body<VECW, 1>(a); }
+extern "C" __global__ void __launch_bounds__(256) nk_fused_grad_steps(const FusedGrad a) { nk_grad_body<1, NK_GRAD_POSITIONS>(a); }
 )NKSRC";
 
 }  // namespace
@@ -601,10 +617,12 @@ extern "C" int nk_fused_compile_grad(nk_ctx* ctx, int32_t dtype, int32_t n_input
     if (!terms || !*terms) return nk_fail(ctx, NK_ERR_BAD_ARG, "nk_fused_compile_grad: empty statement list");
     nk_fused* f = new (std::nothrow) nk_fused();
     if (!f) return nk_fail(ctx, NK_ERR_OOM, "nk_fused_compile_grad: out of host memory");
-    std::string defs = "#define NK_NLEAF " + std::to_string(n_leaves) + "\n#define NK_TERMS " + terms + "\n";
+    std::string defs = "#define NK_GRAD_POSITIONS " + std::to_string(NK_GRAD_POSITIONS) + "\n#define NK_NLEAF " + std::to_string(n_leaves) + "\n#define NK_TERMS " + terms + "\n";
     int st = compile_unit(ctx, "nk_fused_compile_grad", dtype, n_inputs, defs, k_grad_src, &f->lib);
     if (st) { delete f; return st; }
-    cudaError_t e = cudaLibraryGetKernel(&f->kernel, f->lib, "nk_fused_grad_kernel");
+    cudaError_t e = cudaLibraryGetKernel(&f->kernel, f->lib, "nk_fused_grad_one");
+    if (e == cudaSuccess) e = cudaLibraryGetKernel(&f->grad_vec, f->lib, "nk_fused_grad_vec");
+    if (e == cudaSuccess) e = cudaLibraryGetKernel(&f->grad_steps, f->lib, "nk_fused_grad_steps");
     if (e != cudaSuccess) {
         cudaLibraryUnload(f->lib);
         delete f;
@@ -832,8 +850,8 @@ extern "C" int nk_fused_run_grad(nk_ctx* ctx, nk_fused* f, int32_t rank, nk_buf*
         for (int j = 0; j < f->n_in && vec; j++) vec = lane_ok(a.ks[j][n], srcs[j]->ptr, v[j].base, a.ks[j], a.rs[j], 1u << j);
         for (int q = 0; q < n && vec; q++) vec = a.ks0[q] % W == 0;
     }
-    // fewer than four positions of the lowest reduced dim: whole vectors (where possible); otherwise one element per thread
-    if (a.nr > 0 && a.rext[0] >= 4) vec = false;
+    const int form = nk_fused_grad_form(vec ? total / W : 0, a.nr > 0 ? a.rext[0] : 1, ctx->prop.multiProcessorCount);
+    vec = form == NK_GRAD_VEC;
     if (!vec) a.stream_mask = 0;
     a.vec = vec ? W : 1;
     int64_t d = 1;
@@ -841,8 +859,9 @@ extern "C" int nk_fused_run_grad(nk_ctx* ctx, nk_fused* f, int32_t rank, nk_buf*
     a.total = total / a.vec;
     if (a.total == 0) return NK_OK;
     void* params[] = {&a};
-    NK_CUDA(ctx, cudaLaunchKernel(reinterpret_cast<const void*>(f->kernel), dim3(unsigned(nk_grid_for(ctx, a.total, 256, 8))), dim3(256), params, 0, ctx->stream));
-    return nk_after_launch(ctx, "nk_fused_grad_kernel");
+    const cudaKernel_t kernel = form == NK_GRAD_VEC ? f->grad_vec : form == NK_GRAD_STEPS ? f->grad_steps : f->kernel;
+    NK_CUDA(ctx, cudaLaunchKernel(reinterpret_cast<const void*>(kernel), dim3(unsigned(nk_grid_for(ctx, a.total, 256, 8))), dim3(256), params, 0, ctx->stream));
+    return nk_after_launch(ctx, form == NK_GRAD_VEC ? "nk_fused_grad_vec" : form == NK_GRAD_STEPS ? "nk_fused_grad_steps" : "nk_fused_grad_one");
 }
 
 extern "C" int nk_fused_free(nk_fused* f) {

@@ -221,3 +221,27 @@ def test_fused_refuses_what_it_cannot_do(device):
     assert L.lib.nk_fused_compile(device.ctx, L.NK_I32, 1, b"x0", C.byref(h)) == L.NK_ERR_UNSUPPORTED
     assert L.lib.nk_fused_compile(device.ctx, L.NK_F32, 9, b"x0", C.byref(h)) == L.NK_ERR_BAD_ARG
     assert L.lib.nk_fused_free(None) == L.NK_ERR_BAD_ARG
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("shape,positions,kernel", [
+    ([5, 1, 33], 1, "one"), ([5, 1, 33], 3, "one"), ([5, 1, 64], 4, "one"),                             # nothing or little summed
+    ([5, 1, 33], 5, "steps"), ([5, 1, 64], 8, "steps"), ([5, 1, 33], 12, "steps"), ([5, 1, 33], 13, "steps"), ([5, 1, 33], 23, "steps"),
+    ([160, 1, 1024], 1, "vec"), ([160, 1, 1024], 3, "vec"), ([1300, 1, 1024], 9, "vec"),                # enough vectors
+])
+def test_every_form_of_the_fused_gradient(device, dt, shape, positions, kernel):
+    """Extents around the groups of eight positions and the number of vectors each form starts at: the bits of the op-by-op gradient."""
+    rng = np.random.default_rng(positions)
+    full = [shape[0], positions, shape[2]]
+    a, b, e = (Tensor.of(dt, s, rng.uniform(-2.0, 2.0, size=int(np.prod(s))).astype(dt)) for s in (shape, full, full))
+    for t in (a, b):
+        t.set_rqs_gradient(True).to(device)
+    f = Function.of("silu(i0*i1+i1)")
+    f(a, b).backward(e.to(device))
+    fused = device.optimized_operation_of(f, "fused_forms_test")
+    got = fused.gradient(0, e, a, b)
+    assert device.last_kernel() == "nk_fused_grad_" + kernel
+    assert _same_bits(got.items, a.gradient.items)
+    got = fused.gradient(1, e, a, b)   # full shape: never summed
+    assert device.last_kernel() in ("nk_fused_grad_one", "nk_fused_grad_vec") and _same_bits(got.items, b.gradient.items)
+    fused.close()

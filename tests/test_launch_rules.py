@@ -13,6 +13,7 @@ extern "C" void dgemm_parts(int64_t tiles, int64_t k_panels, int64_t sms, int64_
     out[0] = p.splits;
     out[1] = p.kb_per;
 }
+extern "C" int grad_form(int64_t vectors, int64_t positions, int64_t sms) { return nk_fused_grad_form(vectors, positions, sms); }
 """
 
 
@@ -54,3 +55,16 @@ def test_parts_of_f64_products_are_bounded_and_cover_k(rules):
 def test_few_tiles_and_a_long_sum_are_split(rules):
     assert dgemm_parts(rules, 64, 20000, 64)[1] == 16
     assert dgemm_parts(rules, 777, 1023, 515)[1] > 1
+
+
+def test_form_of_a_fused_gradient(rules):
+    """Nothing or little summed: no form that evaluates positions it does not add; many vectors: vectors at any depth."""
+    ONE, VEC, STEPS = 0, 1, 2
+
+    def form(vectors, positions):
+        return rules.grad_form(C.c_int64(vectors), C.c_int64(positions), C.c_int64(148))
+    for positions in (1, 2, 3, 4):
+        assert form(0, positions) == ONE and form(1000, positions) == ONE and form(100_000, positions) == VEC
+    for positions in (5, 7, 8, 9, 1000):
+        assert form(0, positions) == STEPS and form(100_000, positions) == (STEPS if positions >= 8 else VEC)
+    assert all(form(1 << 20, positions) == VEC for positions in (1, 4, 5, 9, 1000))
