@@ -114,34 +114,40 @@ static bool nk_describe_for_tma(const nk_buf* buf, const NkView& v, size_t es, b
 // copy, kernel and release all queue on the context's stream.
 struct StageDims {
     int n_outer;                                   // dims before the last
-    long long rows, base;
-    int width;                                     // extent of the last dim
+    long long base;
+    long long units;                               // segments of all rows
+    int segs;                                      // segments per row
+    long long width;                               // extent of the last dim
     long long sx;                                  // its source stride
     long long ext[NK_MAX_RANK], sstride[NK_MAX_RANK];
     long long pitch;                               // elements per copied row
 };
-// A row per warp and step: one decode of the row index, then coalesced runs, four loads per lane in flight.
+// A segment of a row (up to STAGE_SEG elements) per warp and step: one decode of its place, then coalesced runs, four loads per lane
+// in flight. Segments, so that few long rows keep as many warps busy as many short ones: 2 x 1000003 F32 with a warp per row took 1.6 ms.
 // 16x16x131x127 F32: 13 us; decoding every element with 64-bit divisions: 41.
+constexpr int STAGE_SEG = 1024;
 template <class T>
 __global__ void __launch_bounds__(256) nk_stage_kernel(T* __restrict__ dst, const T* __restrict__ src, const StageDims d) {
     const int lane = threadIdx.x & 31;
     const long long warps = (long long)gridDim.x * 8;
-    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < d.rows; r += warps) {
-        long long rem = r, so = d.base;
+    for (long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); i < d.units; i += warps) {
+        const long long r = d.segs > 1 ? i / d.segs : i, x0 = (i - r * d.segs) * STAGE_SEG;
+        const int left = int(d.width - x0 < STAGE_SEG ? d.width - x0 : STAGE_SEG);
+        long long rem = r, so = d.base + x0 * d.sx;
         for (int k = d.n_outer - 1; k >= 0; k--) {
             const long long q = rem / d.ext[k];
             so += (rem - q * d.ext[k]) * d.sstride[k];
             rem = q;
         }
-        T* out = dst + r * d.pitch;
-        for (int x = lane; x < d.width; x += 128) {
+        T* out = dst + r * d.pitch + x0;
+        for (int x = lane; x < left; x += 128) {
             T v[4];
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (x + 32 * u < d.width) v[u] = src[so + (x + 32 * u) * d.sx];
+                if (x + 32 * u < left) v[u] = src[so + (x + 32 * u) * d.sx];
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (x + 32 * u < d.width) out[x + 32 * u] = v[u];
+                if (x + 32 * u < left) out[x + 32 * u] = v[u];
         }
     }
 }
@@ -159,17 +165,18 @@ static int nk_stage_operand(nk_ctx* ctx, int dtype, const nk_buf* src, const NkV
     memset(&d, 0, sizeof(d));
     d.n_outer = rank - 1;
     d.base = v.base;
-    d.width = int(v.shape[X]);
+    d.width = v.shape[X];
+    d.segs = int((d.width + STAGE_SEG - 1) / STAGE_SEG);
+    d.units = d.segs;
     d.sx = v.estride[X];
     d.pitch = pitch;
     out->view = v;
     out->view.base = 0;
-    d.rows = 1;
     int64_t ds = 1;
     for (int k = rank - 1; k >= 0; k--) {
         d.ext[k] = v.shape[k];
         d.sstride[k] = v.estride[k];
-        if (k != X) d.rows *= v.shape[k];
+        if (k != X) d.units *= v.shape[k];
         out->view.estride[k] = ds;
         ds *= (k == X) ? pitch : v.shape[k];
     }
@@ -183,7 +190,7 @@ static int nk_stage_operand(nk_ctx* ctx, int dtype, const nk_buf* src, const NkV
     out->buf.n_elems = ds;
     out->buf.owned = false;
     out->used = true;
-    const int grid = nk_grid_for(ctx, d.rows, 8, 16);
+    const int grid = nk_grid_for(ctx, d.units, 8, 16);
     if (dtype == NK_F32) nk_stage_kernel<float><<<grid, 256, 0, ctx->stream>>>(static_cast<float*>(ptr), static_cast<const float*>(src->ptr), d);
     else nk_stage_kernel<double><<<grid, 256, 0, ctx->stream>>>(static_cast<double*>(ptr), static_cast<const double*>(src->ptr), d);
     return nk_after_launch(ctx, "nk_stage_kernel");

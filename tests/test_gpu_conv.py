@@ -4,10 +4,12 @@ dense / sliced / strided / column-major / permuted views, F32 and F64, forward a
 Tolerances (stated by the task): relative error <= 1e-5 (F32) / <= 1e-12 (F64). "Relative" is taken against the
 magnitude the sum can reach, |a|.|b| summed the same way (computed by the oracle on absolute values): that is
 the bound that holds for any summation order; a plain max-norm relative check is applied as well."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from helpers import gpu_conv, rand_view
+from helpers import DevArray, cfgp, gpu_conv, rand_view
 from neureka_b200 import _lib as L
 from neureka_b200.ndconf import Layout, NDConfiguration as ND
 
@@ -434,3 +436,48 @@ def test_contractions_of_the_multiply_add_family(device, dt, mkn, order):
     # rounding of a sum of k products in any order: (k + splits) half units in the last place of sum|a||b|
     bound = (k + 16) * float(np.finfo(dt).eps) / 2 * (np.abs(A) @ np.abs(B))
     assert np.all(np.abs(runs[0].reshape(m, n) - A @ B) <= bound)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("width", [1024 + 5, 2 * 1024 + 4 + 3, 300_003])
+def test_gradients_of_few_long_odd_rows(device, dt, width):
+    """Rows of several segments of the padded copy (whole, and with remainders of one and a few elements): the numbers of the gather
+    family, and of the same tensors as a view with gaps."""
+    rng = np.random.default_rng(width)
+    sa, sb = [3, width], [1, 5]
+    so = [3, width - 4]
+    a, b, e = (rng.standard_normal(int(np.prod(s))).astype(dt) for s in (sa, sb, so))
+    c0, c1, c2 = ND.of_shape(so), ND.of_shape(sa), ND.of_shape(sb)
+    bound = 8 * (1e-5 if dt == np.float32 else 1e-12)
+    grad = gpu_conv(device, np.full(c1.size, 777.0, dtype=dt), c1, b, c2, e, c0, d=0)
+    assert device.last_conv_path() == L.NK_CONV_TMA
+    want = gpu_conv(device, np.zeros(c1.size, dtype=dt), c1, b, c2, e, c0, d=0, path=L.NK_CONV_GENERIC)
+    assert np.abs(grad - want).max() <= bound * np.abs(want).max()
+    par = np.zeros([3, 2 * (width - 4) + 1], dtype=dt)
+    par[:, 1::2] = e.reshape(so)
+    cpar = ND.of_shape(list(par.shape)).sliced(so, [0, 1], [1, 2])
+    assert np.array_equal(gpu_conv(device, np.full(c1.size, 777.0, dtype=dt), c1, b, c2, par.ravel(), cpar, d=0), grad)
+    if 3 * (width - 4) >= 65536:
+        gk = gpu_conv(device, np.full(5, 777.0, dtype=dt), c2, a, c1, e, c0, d=0)
+        assert device.last_conv_path() == L.NK_CONV_TMA
+        windows = [a.reshape(sa)[:, i:i + width - 4].ravel().astype(np.float64) for i in range(5)]
+        for i, w in enumerate(windows):   # whatever the order of the sum
+            assert abs(gk[i] - w @ e) <= bound / 8 * (np.abs(w) @ np.abs(e))
+
+
+def test_the_padded_copy_of_few_long_rows_uses_the_whole_chip(device):
+    """The image gradient of two rows of a million elements of odd pitch against the same at a pitch a tensor map takes (no copy):
+    a copy by one warp per row took 60 times as long as the gradient itself."""
+    def best_ms(width):
+        shapes = [2, width], [1, 5], [2, width - 4]
+        g, k, e = (DevArray(device, np.ones(int(np.prod(s)), dtype=np.float32)) for s in shapes)
+        (k0, p0), (k1, p1), (k2, p2) = (cfgp(ND.of_shape(s)) for s in shapes)
+        ms, best = C.c_float(), 1e30
+        for _ in range(6):
+            L.check(L.lib.nk_timer_begin(device.ctx), device.ctx)
+            for _ in range(5):
+                L.check(L.lib.nk_conv(device.ctx, L.NK_F32, 2, g.buf, p0, k.buf, p1, e.buf, p2, 0), device.ctx)
+            L.check(L.lib.nk_timer_end(device.ctx, C.byref(ms)), device.ctx)
+            best = min(best, ms.value)
+        return best
+    assert best_ms(1_000_003) < 8 * best_ms(1_000_004)
