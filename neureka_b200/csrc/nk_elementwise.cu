@@ -4,6 +4,7 @@
 // Compiled with -fmad=false (see nk_scalarfun.cuh).
 
 #include "nk_ew_kernels.cuh"
+#include "nk_launch_rules.h"
 #include "nk_ptx.cuh"
 
 using namespace nkew;
@@ -226,11 +227,13 @@ __global__ void __launch_bounds__(256) nk_fill_fun_kernel(T* __restrict__ out, E
 //   * nk_sum_rows_kernel (contiguous, 16-byte aligned): a warp requests 32 whole tiles with 16-byte asynchronous copies, into rows
 //     padded by 16 bytes, and lane t then adds row t. The copies need no registers: twelve warps' 16 KB each are in flight per
 //     SM. 2^26 F32 elements: 46 us (40 is the floor); one tile per warp, one lane adding: 487.
-//   * nk_sum_tiles_kernel (any view): the same through registers, 16 elements of every tile at a time.
-//   * nk_sum_last_kernel: at most 128 tiles, i.e. the last two levels of any sum (or all of a sum of up to 2^14 elements) in
+//   * nk_sum_tiles_kernel (any view, many tiles): the same through registers, 16 elements of every tile at a time.
+//   * nk_sum_warp_kernel (any view): a tile per warp, staged by all lanes and added by one -- a thirty-second of the adders, but 32 times
+//     the warps, which is what fewer tiles than the chip has lanes need (1000 x 1000 F32, a slice: 20 us, in groups of 32 tiles 83).
+//   * nk_sum_last_kernel: at most 32 tiles, i.e. the last two levels of any sum (or all of a sum of up to 2^12 elements) in
 //     one CTA: a warp stages a tile, one lane adds it; one lane then adds the tile sums.
 struct SumView {
-    int nd;                       // merged dims
+    int nd;                       // merged dims (0: contiguous, from the pointer on; not for nk_sum_tiles_kernel)
     int64_t div[NK_MAX_RANK], s[NK_MAX_RANK];
     int64_t base;
 };
@@ -239,6 +242,7 @@ __device__ __forceinline__ int64_t sum_offset(const SumView& v, int64_t i) {
     for (int j = 0; j < v.nd; j++) { const int64_t idx = i / v.div[j]; i -= idx * v.div[j]; src += idx * v.s[j]; }
     return src;
 }
+__device__ __forceinline__ int64_t sum_place(const SumView& v, int64_t i) { return v.nd == 0 ? i : sum_offset(v, i); }
 template <class T> struct SumRows {
     static constexpr int VPT = 128 * int(sizeof(T)) / 16;        // 16-byte vectors per tile
     static constexpr int PITCH = 128 + 16 / int(sizeof(T));      // elements per padded row
@@ -328,26 +332,39 @@ __global__ void __launch_bounds__(128) nk_sum_tiles_kernel(const T* __restrict__
     }
 }
 template <class T>
-__global__ void __launch_bounds__(1024) nk_sum_last_kernel(const T* __restrict__ in, const SumView v, int n, T* __restrict__ out) {
-    __shared__ T tile[32][128 + 1];
-    __shared__ T part[128];
+__global__ void __launch_bounds__(128) nk_sum_warp_kernel(const T* __restrict__ in, const SumView v, int64_t n, T* __restrict__ out, int64_t n_tiles) {
+    __shared__ T tile[4][128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = (n + 127) / 128;
-    for (int t = warp; t < n_tiles; t += 32) {
-        const int off = t * 128;
-        const int lim = off + 128 < n ? 128 : n - off;
-        for (int k = lane; k < lim; k += 32) tile[warp][k] = in[sum_offset(v, off + k)];
+    for (int64_t t = int64_t(blockIdx.x) * 4 + warp; t < n_tiles; t += int64_t(gridDim.x) * 4) {
+        const int64_t off = t * 128;
+        const int lim = off + 128 < n ? 128 : int(n - off);
+        for (int k = lane; k < lim; k += 32) tile[warp][k] = in[sum_place(v, off + k)];
         __syncwarp();
         if (lane == 0) {
             T value = 0;
             for (int k = 0; k < lim; k++) value += tile[warp][k];
-            part[t] = value;
+            out[t] = value;
         }
         __syncwarp();
+    }
+}
+template <class T>
+__global__ void __launch_bounds__(1024) nk_sum_last_kernel(const T* __restrict__ in, const SumView v, int n, T* __restrict__ out) {
+    __shared__ T tile[NK_SUM_LAST / 128][128];
+    __shared__ T part[NK_SUM_LAST / 128];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, off = warp * 128;   // a warp per tile
+    const int lim = off + 128 < n ? 128 : n - off;
+    for (int k = lane; k < lim; k += 32) tile[warp][k] = in[sum_place(v, off + k)];
+    __syncwarp();
+    if (lane == 0) {
+        T value = 0;
+        for (int k = 0; k < lim; k++) value += tile[warp][k];
+        part[warp] = value;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         // a single tile is the result; several are one more tile, added in order from 0
+        const int n_tiles = int(blockDim.x >> 5);
         T value = 0;
         if (n_tiles == 1) value = part[0];
         else for (int k = 0; k < n_tiles; k++) value += part[k];
@@ -486,10 +503,14 @@ static int sum_impl(nk_ctx* ctx, const T* in, const EwPlan& p, int64_t n, T* out
     v.nd = p.nd;
     v.base = p.b0;
     for (int k = 0; k < p.nd; k++) { v.div[k] = p.div[k]; v.s[k] = p.s0[k]; }
-    bool rows = p.nd == 1 && p.row_major && p.s0[0] == 1 && aligned16(in + p.b0);
-    if (rows) { in += p.b0; v.base = 0; }
+    if (p.nd == 1 && p.row_major && p.s0[0] == 1) {   // contiguous
+        in += p.b0;
+        v.nd = 0;
+        v.base = 0;
+    }
+    bool rows = v.nd == 0 && aligned16(in);
     T *bufA = nullptr, *bufB = nullptr;
-    if (n > 16384) {
+    if (n > NK_SUM_LAST) {
         const int64_t n1 = (n + 127) / 128, n2 = (n1 + 127) / 128;
         void* scratch = nullptr;
         int st = nk_scratch(ctx, size_t(n1 + n2 + 16) * sizeof(T), &scratch);
@@ -501,25 +522,34 @@ static int sum_impl(nk_ctx* ctx, const T* in, const EwPlan& p, int64_t n, T* out
     const T* src = in;
     int64_t cur = n;
     T* dst = bufA;
-    while (cur > 16384) {
+    while (cur > NK_SUM_LAST) {
         const int64_t tiles = (cur + 127) / 128;
-        if (rows) {
+        const char* name;
+        if (rows && nk_sum_by_rows(tiles, ctx->prop.multiProcessorCount)) {
+            name = "nk_sum_rows_kernel";
             using C = SumRows<T>;
             nk_sum_rows_kernel<T><<<nk_grid_for(ctx, (tiles + 31) / 32, C::WARPS, 12), C::WARPS * 32, C::SMEM, ctx->stream>>>(src, cur, dst, tiles);
-        } else {
+        } else if (!rows && nk_sum_by_groups(tiles, v.nd, ctx->prop.multiProcessorCount)) {
+            name = "nk_sum_tiles_kernel";
+            if (v.nd == 0) {   // (asking for it in the kernel costs views 5 %)
+                v.nd = 1;
+                v.div[0] = v.s[0] = 1;
+            }
             nk_sum_tiles_kernel<T><<<nk_grid_for(ctx, (tiles + 31) / 32, 4, 16), 128, 0, ctx->stream>>>(src, v, cur, dst, tiles);
+        } else {
+            name = "nk_sum_warp_kernel";
+            nk_sum_warp_kernel<T><<<nk_grid_for(ctx, tiles, 4, 16), 128, 0, ctx->stream>>>(src, v, cur, dst, tiles);
         }
-        const int st = nk_after_launch(ctx, "nk_sum_tiles_kernel");
+        const int st = nk_after_launch(ctx, name);
         if (st) return st;
         src = dst;
         rows = true;   // the next levels are dense
-        v.nd = 1;
+        v.nd = 0;
         v.base = 0;
-        v.div[0] = v.s[0] = 1;
         cur = tiles;
         dst = (dst == bufA) ? bufB : bufA;
     }
-    nk_sum_last_kernel<T><<<1, 1024, 0, ctx->stream>>>(src, v, int(cur), out_elem);
+    nk_sum_last_kernel<T><<<1, int((cur + 127) / 128) * 32, 0, ctx->stream>>>(src, v, int(cur), out_elem);
     return nk_after_launch(ctx, "nk_sum_last_kernel");
 }
 

@@ -51,3 +51,16 @@ inline int nk_fused_grad_form(int64_t vectors, int64_t positions, int64_t sms) {
     if (vectors >= sms * 256) return NK_GRAD_VEC;
     return positions > NK_GRAD_POSITIONS / 2 ? NK_GRAD_STEPS : NK_GRAD_ONE;
 }
+
+// ---- sums: what adds the tiles of 128 elements ----------------------------------------------------------------------------
+constexpr int64_t NK_SUM_LAST = 4096;   // elements that one CTA adds by itself: a tile per warp (16384, four tiles per warp: 18 us, two launches 10)
+
+// Contiguous and 16-byte aligned: 32 tiles per warp through asynchronous copies where a warp per tile would take more than 40 warps per SM.
+// F32, us, rows / warps: 300000 elements 10.3 / 8.2, 600000 14.3 / 12.3, 2^20 13.3 / 14.4, 2^21 13.3 / 16.4, 2^23 18.5 / 33.
+inline bool nk_sum_by_rows(int64_t tiles, int64_t sms) { return tiles >= sms * 40; }
+
+// A view that 16-byte copies do not fit: 32 tiles per warp with an adder per lane (true), or a tile per warp with one adder. A group takes
+// 60 to 100 us of dependent loads however few there are, a warp (64 per SM) about 8 us per tile, more where several dims have to be
+// taken apart. F32, us, groups / warps: 2^20 elements from an odd address 68 / 18, 12.6 M 74 / 72, 16.8 M 78 / 90, 33.6 M 154 / 208; a slice of
+// 1000 x 1000 83 / 21; 300 x 300 x 300 turned 268 / 242 (F64 405 / 270), 400 x 400 x 400 turned 545 / 627 (734 / 742).
+inline bool nk_sum_by_groups(int64_t tiles, int merged_dims, int64_t sms) { return tiles >= sms * 64 * (merged_dims <= 2 ? 12 : 24); }

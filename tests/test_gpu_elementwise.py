@@ -331,3 +331,43 @@ def test_value_and_derivative_in_one_pass(device, dt, fun):
         for got, d in ((D.read(), -1), (E.read(), 0)):
             assert np.array_equal(got, gpu_unary(device, L.FUN[fun], np.zeros(n, dtype=dt), dense, x, conf, d=d), equal_nan=True), (fun, d)
     assert L.lib.nk_unary_both(device.ctx, 99, S.nk_dtype, 1, D.buf, p0, E.buf, p0, S.buf, p0) == L.NK_ERR_BAD_ARG
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n,kernels", [(4096, 1), (4097, 2), (148 * 40 * 128 - 127, 3), (148 * 40 * 128 + 5, 3), (148 * 64 * 12 * 128 - 100, 3), (148 * 64 * 12 * 128 + 77, 3)])
+def test_sums_on_either_side_of_every_rule(device, oracle, dt, n, kernels):
+    """One CTA and two levels; a warp per tile and groups of 32 tiles, contiguous and through views (an odd start, a gap after every
+    element, two dims): CPUSum's bits. The sizes are the rules' for 148 SMs."""
+    rng = np.random.default_rng(n)
+    host = rng.standard_normal(2 * n + 1).astype(dt)
+    S, O = DevArray(device, host), DevArray(device, np.zeros(1, dtype=dt))
+    parent = ND.of_shape([2 * n + 1])
+    cases = [(parent.sliced([n], [0], [1]), host[:n]), (parent.sliced([n], [1], [1]), host[1:n + 1]), (parent.sliced([n], [1], [2]), host[1::2][:n])]
+    rows = n // 1000
+    if rows >= 2:   # rows of 1000 out of 1500
+        cases.append((ND.of_shape([rows, 1500]).sliced([rows, 1000], [0, 3], [1, 1]), host[:rows * 1500].reshape(rows, 1500)[:, 3:1003].reshape(-1)))
+    for conf, items in cases:
+        k, p = cfgp(conf)
+        before = device.launch_count()
+        L.check(L.lib.nk_sum(device.ctx, S.nk_dtype, conf.rank, S.buf, p, O.buf, 0), device.ctx)
+        if items.size == n:
+            assert device.launch_count() - before == kernels
+        assert O.read()[0] == dt(oracle.cpu_sum(np.ascontiguousarray(items)))
+
+
+def test_a_sum_through_a_view_takes_about_as_long_as_the_contiguous_one(device):
+    """300000 elements from an odd start: with 32 tiles per warp the few warps' dependent loads took five times as long."""
+    n = 300_000
+    S, O = DevArray(device, np.ones(n + 1, dtype=np.float32)), DevArray(device, np.zeros(1, dtype=np.float32))
+    ms, took = C.c_float(), []
+    for start in (0, 1):
+        k, p = cfgp(ND.of_shape([n + 1]).sliced([n], [start], [1]))
+        best = 1e30
+        for _ in range(6):
+            L.check(L.lib.nk_timer_begin(device.ctx), device.ctx)
+            for _ in range(20):
+                L.check(L.lib.nk_sum(device.ctx, L.NK_F32, 1, S.buf, p, O.buf, 0), device.ctx)
+            L.check(L.lib.nk_timer_end(device.ctx, C.byref(ms)), device.ctx)
+            best = min(best, ms.value)
+        took.append(best)
+    assert took[1] < 2.5 * took[0]

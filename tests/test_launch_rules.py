@@ -13,6 +13,8 @@ extern "C" void dgemm_parts(int64_t tiles, int64_t k_panels, int64_t sms, int64_
     out[0] = p.splits;
     out[1] = p.kb_per;
 }
+extern "C" int sum_by_groups(int64_t tiles, int merged_dims, int64_t sms) { return nk_sum_by_groups(tiles, merged_dims, sms); }
+extern "C" int64_t sum_last() { return NK_SUM_LAST; }
 extern "C" int grad_form(int64_t vectors, int64_t positions, int64_t sms) { return nk_fused_grad_form(vectors, positions, sms); }
 """
 
@@ -68,3 +70,12 @@ def test_form_of_a_fused_gradient(rules):
     for positions in (5, 7, 8, 9, 1000):
         assert form(0, positions) == STEPS and form(100_000, positions) == (STEPS if positions >= 8 else VEC)
     assert all(form(1 << 20, positions) == VEC for positions in (1, 4, 5, 9, 1000))
+
+
+def test_sums_of_views_go_by_groups_only_where_groups_fill_the_chip(rules):
+    rules.sum_last.restype = C.c_int64
+    assert rules.sum_last() == 32 * 128                  # a tile per warp of one CTA
+    for dims in range(0, 9):
+        for n in (8192, 16385, 300_000, 1_000_000, 1 << 21, 8_000_000):
+            assert not rules.sum_by_groups(C.c_int64(-(-n // 128)), C.c_int(dims), C.c_int64(148)), (n, dims)
+        assert rules.sum_by_groups(C.c_int64((1 << 25) // 128), C.c_int(dims), C.c_int64(148))
