@@ -143,7 +143,9 @@ int nk_binary(nk_ctx* ctx, int32_t op, int32_t dtype, int32_t rank,
 int nk_unary(nk_ctx* ctx, int32_t fun, int32_t dtype, int32_t rank,
              nk_buf* drn, const int32_t* cfg0, nk_buf* src, const int32_t* cfg1, int32_t d);
 
-/* drain = f(src) and ddrain = f'(src) in one pass over src: what nk_unary gives with d < 0 and d >= 0, bit for bit. */
+/* drain = f(src) and ddrain = f'(src): what nk_unary gives with d < 0 and d >= 0, bit for bit; one pass over src where all three are
+ * contiguous and 16-byte aligned. One of the drains may be src itself (the same view of the same memory); apart from that no two of the
+ * three may overlap. */
 int nk_unary_both(nk_ctx* ctx, int32_t fun, int32_t dtype, int32_t rank,
                   nk_buf* drn, const int32_t* cfg0, nk_buf* ddrn, const int32_t* cfgd, nk_buf* src, const int32_t* cfg1);
 

@@ -42,7 +42,7 @@ int launch_scalar(nk_ctx* ctx, int op, int d, T value, T* out, const T* in, cons
 // next vector is requested before this one's arithmetic, as in nk_ew_linear_kernel. tanh over 2^26 F32: its F64 arithmetic (about
 // 135 us) and 12 bytes per element (121 us) bound the pass, which takes 170; the two separate ones took 136 + 150.
 template <class T, class F0, class F1>
-__global__ void __launch_bounds__(256) nk_ew_both_kernel(T* __restrict__ out, T* __restrict__ der, const T* __restrict__ a, int64_t n, F0 f0, F1 f1) {
+__global__ void __launch_bounds__(256) nk_ew_both_kernel(T* out, T* der, const T* a, int64_t n, F0 f0, F1 f1) {   // (either drain may be the source)
     using V = typename Vec4<T>::type;
     constexpr int N = Vec4<T>::N;
     const int64_t nvec = n / N, stride = int64_t(gridDim.x) * blockDim.x, tid = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -58,8 +58,9 @@ __global__ void __launch_bounds__(256) nk_ew_both_kernel(T* __restrict__ out, T*
         cur = nxt;
     }
     for (int64_t i = nvec * N + tid; i < n; i += stride) {
-        out[i] = f0(a[i], T(0));
-        der[i] = f1(a[i], T(0));
+        const T x = a[i];
+        out[i] = f0(x, T(0));
+        der[i] = f1(x, T(0));
     }
 }
 template <class T, class F0, class F1>
@@ -74,8 +75,14 @@ int unary_both(nk_ctx* ctx, int fun, T* out, T* der, const T* in, const EwPlan& 
     const bool dense = p.row_major && pd.row_major && p.nd == 1 && pd.nd == 1 && p.s0[0] == 1 && p.s1[0] == 1 && pd.s0[0] == 1 &&
                        aligned16(out + p.b0) && aligned16(in + p.b1) && aligned16(der + pd.b0);
     if (!dense) {
-        const int st = launch_unary<T>(ctx, fun, false, out, in, p);
-        return st ? st : launch_unary<T>(ctx, fun, true, der, in, pd);
+        // the drain that is the source itself is written last
+        const bool derivative_last = der + pd.b0 == in + pd.b1;
+        if (derivative_last) {
+            const int st = launch_unary<T>(ctx, fun, false, out, in, p);
+            return st ? st : launch_unary<T>(ctx, fun, true, der, in, pd);
+        }
+        const int st = launch_unary<T>(ctx, fun, true, der, in, pd);
+        return st ? st : launch_unary<T>(ctx, fun, false, out, in, p);
     }
     out += p.b0; der += pd.b0; in += p.b1;
 #define NK_BOTH_CASE(FUN) case FUN: return launch_both<T>(ctx, out, der, in, p.total, UnaryFix<T, FUN, false>{}, UnaryFix<T, FUN, true>{});

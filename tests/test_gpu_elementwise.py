@@ -371,3 +371,24 @@ def test_a_sum_through_a_view_takes_about_as_long_as_the_contiguous_one(device):
             best = min(best, ms.value)
         took.append(best)
     assert took[1] < 2.5 * took[0]
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("fun", ["tanh", "gelu", "quad", "softplus"])
+@pytest.mark.parametrize("start,spread", [(0, 1), (1, 1), (1, 2)])
+def test_value_and_derivative_with_a_drain_that_is_the_source(device, dt, fun, start, spread):
+    """In place, on the one-pass route (aligned and contiguous) and on the two-launch route: both results are of the source as it was."""
+    n = 1027
+    host = _inputs(np.random.default_rng(71), 2 * n + 1, dt, fun)
+    conf, dense = ND.of_shape([2 * n + 1]).sliced([n], [start], [spread]), ND.of_shape([n])
+    (k, p), (kd, pd) = cfgp(conf), cfgp(dense)
+    f = L.FUN[fun]
+    items = host[start:start + (n - 1) * spread + 1:spread].copy()
+    value, deriv = (gpu_unary(device, f, np.zeros(n, dtype=dt), dense, items, dense, d=d) for d in (-1, 0))
+    for value_in_place in (True, False):
+        S, O = DevArray(device, host), DevArray(device, np.zeros(n, dtype=dt))
+        drains = (S.buf, p, O.buf, pd) if value_in_place else (O.buf, pd, S.buf, p)
+        L.check(L.lib.nk_unary_both(device.ctx, f, S.nk_dtype, 1, *drains, S.buf, p), device.ctx)
+        inside, outside = (value, deriv) if value_in_place else (deriv, value)
+        assert np.array_equal(S.read()[start:start + (n - 1) * spread + 1:spread], inside)
+        assert np.array_equal(O.read(), outside)
