@@ -88,6 +88,7 @@ int unary_both(nk_ctx* ctx, int fun, T* out, T* der, const T* in, const EwPlan& 
 #define NK_BOTH_CASE(FUN) case FUN: return launch_both<T>(ctx, out, der, in, p.total, UnaryFix<T, FUN, false>{}, UnaryFix<T, FUN, true>{});
     switch (fun) {
         NK_BOTH_CASE(NK_FUN_TANH) NK_BOTH_CASE(NK_FUN_SIG) NK_BOTH_CASE(NK_FUN_SILU) NK_BOTH_CASE(NK_FUN_GELU) NK_BOTH_CASE(NK_FUN_RELU)
+        NK_BOTH_CASE(NK_FUN_SOFTPLUS)
         default: break;
     }
 #undef NK_BOTH_CASE

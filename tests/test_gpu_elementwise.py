@@ -392,3 +392,29 @@ def test_value_and_derivative_with_a_drain_that_is_the_source(device, dt, fun, s
         inside, outside = (value, deriv) if value_in_place else (deriv, value)
         assert np.array_equal(S.read()[start:start + (n - 1) * spread + 1:spread], inside)
         assert np.array_equal(O.read(), outside)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+def test_value_and_derivative_in_one_pass_take_no_longer_than_two(device, dt):
+    """Every function at 2^24 elements: a function that the one-pass kernel looks up at run time had the registers of all of them, which
+    cost softplus 18 %."""
+    n = 1 << 24
+    S, D, E = (DevArray(device, np.full(n, 0.7, dtype=dt)) for _ in range(3))
+    k, p = cfgp(ND.of_shape([n]))
+    ms = C.c_float()
+
+    def best(calls):
+        took = 1e30
+        for _ in range(6):
+            L.check(L.lib.nk_timer_begin(device.ctx), device.ctx)
+            for _ in range(3):
+                for call in calls:
+                    L.check(call(), device.ctx)
+            L.check(L.lib.nk_timer_end(device.ctx, C.byref(ms)), device.ctx)
+            took = min(took, ms.value)
+        return took
+    for fun in L.FUN_IDS:
+        f = L.FUN[fun]
+        one = best([lambda: L.lib.nk_unary_both(device.ctx, f, S.nk_dtype, 1, D.buf, p, E.buf, p, S.buf, p)])
+        two = best([lambda: L.lib.nk_unary(device.ctx, f, S.nk_dtype, 1, D.buf, p, S.buf, p, -1), lambda: L.lib.nk_unary(device.ctx, f, S.nk_dtype, 1, E.buf, p, S.buf, p, 0)])
+        assert one <= 1.08 * two, (fun, one, two)
