@@ -418,3 +418,15 @@ def test_value_and_derivative_in_one_pass_take_no_longer_than_two(device, dt):
         one = best([lambda: L.lib.nk_unary_both(device.ctx, f, S.nk_dtype, 1, D.buf, p, E.buf, p, S.buf, p)])
         two = best([lambda: L.lib.nk_unary(device.ctx, f, S.nk_dtype, 1, D.buf, p, S.buf, p, -1), lambda: L.lib.nk_unary(device.ctx, f, S.nk_dtype, 1, E.buf, p, S.buf, p, 0)])
         assert one <= 1.08 * two, (fun, one, two)
+
+
+@pytest.mark.parametrize("dt,rows,kernel", [(np.float32, 1001, "nk_ew_flat32_kernel"), (np.float64, 1001, "nk_ew_flat32_kernel"), (np.float64, 4211, "nk_ew_flat_kernel")])
+def test_drains_whose_rows_are_not_contiguous(device, dt, rows, kernel):
+    """A transposed drain within and beyond the size of L2 (126 MB): exact, on the form that is faster there."""
+    cols = 4099
+    rng = np.random.default_rng(73)
+    a, b = (rng.standard_normal(rows * cols).astype(dt) for _ in range(2))
+    dense, turned = ND.of_shape([rows, cols]), ND.of_shape([cols, rows]).reshaped([1, 0])
+    got = gpu_call3(L.lib.nk_binary, device, L.OPS["*"], np.zeros(rows * cols, dtype=dt), turned, a, dense, b, dense)
+    assert device.last_kernel() == kernel
+    assert np.array_equal(got.reshape(cols, rows).T.reshape(-1), a * b)
