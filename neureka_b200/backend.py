@@ -140,8 +140,12 @@ class CudaBiElementwise(ImplementationFor):
             raise ValueError("The element-wise operation requires at least two arguments and one output!")
         dev = call.device
         t0, t1, t2 = call.input(0), call.input(1), call.input(2)
-        # (the reference actualises virtual operands first, CPUBiElementWise.java:59-60; the kernel reads their one element through
-        # a configuration that maps every index to it, which saves filling and re-reading an array of the drain's size)
+        # A virtual operand stays one element: the kernel reads it through a configuration that maps every index to it. Only the drain
+        # itself has to become a whole tensor (CPUBiElementWise.java:59-60 does that for every operand); a view of a virtual tensor
+        # cannot be one and is refused.
+        for t in (t1, t2):
+            if t.is_virtual and (t is t0 or t.is_slice()):
+                t.set_is_virtual(False)
         dt = _same_type(call, 3)
         k0, c0 = _cfg(t0); k1, c1 = _cfg_virtual(t1); k2, c2 = _cfg_virtual(t2)
         L.check(L.lib.nk_binary(dev.ctx, self.op, dt, t0.rank, t0._data.buf, c0, t1._data.buf, c1, t2._data.buf, c2, call.deriv_idx), dev.ctx)

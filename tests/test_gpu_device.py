@@ -277,3 +277,23 @@ def test_bounded_wait_runs_out_and_is_reported(device):
     assert np.all(out == 3.0)
     L.lib.nk_free(device.ctx, buf)
     assert L.lib.nk_probe_wait_timeout(device.ctx, 0, None) == L.NK_ERR_BAD_ARG
+
+
+def test_a_virtual_operand_that_is_the_drain(device):
+    """An elementwise call in place on a virtual tensor: it becomes a whole tensor first, as the drain of any call is one; any other virtual
+    operand stays one element, and a view of a virtual tensor, which cannot become a whole tensor, is refused."""
+    from neureka_b200 import backend as Bk
+    from neureka_b200.backend import ExecutionCall
+    add = Bk.backend().implementation_for("+", Bk.BI_ELEMENTWISE)
+    b_h = np.arange(12, dtype=np.float32)
+    for position in (0, 1):
+        t, b = Tensor.of(np.float32, [3, 4], 2.0).to(device), Tensor.of(np.float32, [3, 4], b_h).to(device)
+        operands = [t, b] if position == 0 else [b, t]
+        assert add.run(ExecutionCall([t, *operands], "+", device)) is t
+        assert not t.is_virtual and np.array_equal(t.items, b_h + 2)
+        v, out = Tensor.of(np.float32, [3, 4], 5.0).to(device), Tensor.of(np.float32, [3, 4], b_h).to(device)
+        add.run(ExecutionCall([out, *([v, b] if position == 0 else [b, v])], "+", device))
+        assert v.is_virtual and np.array_equal(out.items, b_h + 5)
+        view = Tensor.of(np.float32, [4, 3], 5.0).to(device).permute(1, 0)
+        with pytest.raises(ValueError):
+            add.run(ExecutionCall([out, *([view, b] if position == 0 else [b, view])], "+", device))
