@@ -77,6 +77,11 @@ def _zeros_view(dev, dtype, shape) -> Tensor:
     return t
 
 
+def _is_whole(t: Tensor) -> bool:
+    """A tensor of its own in row-major order, which can be handed on or viewed in another shape: not a view, not one virtual element."""
+    return not t.is_virtual and not t.is_slice() and t.ndconf.is_simple()
+
+
 def _record_operator(sym: str, a: Tensor, b: Tensor, out: Tensor) -> None:
     algo = F.choose_algorithm(a, b)
     parents = []
@@ -94,8 +99,8 @@ def _record_operator(sym: str, a: Tensor, b: Tensor, out: Tensor) -> None:
             mine, oth = (fa, fb) if d == 0 else (fb, fa)
             if sym in ("+", "-"):
                 def action(err, mine=mine, dtype=oth.dtype, shape=oth.shape, d=d, sym=sym):
-                    if (sym == "+" or d == 0) and err.shape == mine.shape and not err.is_virtual:
-                        return err   # nothing is summed: the kernel would copy the error (82 us of a step over 2^26 elements)
+                    if (sym == "+" or d == 0) and err.shape == mine.shape and _is_whole(err):
+                        return err   # nothing is summed: the kernel would copy the error (82 us for 2^26 elements)
                     return _reshape_like(_broadcast_reduce(L.OPS[sym], mine, _zeros_view(err.device, dtype, shape), err, d), mine)
                 parents.append((t, action))
             elif sym == "*":
@@ -228,7 +233,7 @@ def _accumulate(t: Tensor, err: Tensor, owned: bool = False) -> None:
     nobody else holds (`owned`) becomes the gradient itself; any other is copied -- a launch and a pass over the tensor that
     a training step pays per parameter."""
     if t.gradient is None:
-        if owned and err.shape == t.shape and err.dtype == t.dtype and not err.is_virtual and not err.is_slice() and err.ndconf.is_simple():
+        if owned and err.shape == t.shape and err.dtype == t.dtype and _is_whole(err):
             err.is_intermediate = False
             t.gradient = err
             return

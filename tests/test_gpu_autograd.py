@@ -333,3 +333,20 @@ def test_gradients_are_tensors_of_their_own(device):
     w = Tensor.of(np.float32, [4, 35], e_h).set_rqs_gradient(True).to(device)
     (w + z).backward(e)   # the caller's error reaches w unchanged: copied
     assert w.gradient._data is not e._data and np.array_equal(w.gradient.numpy(), e.numpy())
+
+
+@pytest.mark.parametrize("op", ["+", "-"])
+def test_an_error_that_is_a_view_reaches_a_lower_rank_operand(device, op):
+    """A sum of a vector and a one-row matrix sums nothing in its backward pass; an error that is a slice, a spread or a transposed view
+    still arrives in the vector's own shape."""
+    rng = np.random.default_rng(5)
+    f = Function.of(f"i0 {op} i1")
+    wide = rng.standard_normal((3, 9)).astype(np.float32)
+    w = Tensor.of(np.float32, [3, 9], wide).to(device)
+    column = Tensor.of(np.float32, [5, 1], wide[0, :5]).to(device)
+    for e, want in ((w[1:2, 0:9:2], wide[1, ::2]), (w[2:3, 3:8], wide[2, 3:8]), (column.permute(1, 0), wide[0, :5])):
+        n = want.size
+        a, b = (Tensor.of(np.float32, s, np.arange(n)).set_rqs_gradient(True).to(device) for s in ([n], [1, n]))
+        f(a, b).backward(e)
+        assert a.gradient.shape == (n,) and np.array_equal(a.gradient.items, want)
+        assert np.array_equal(b.gradient.items, want if op == "+" else -want)
