@@ -191,6 +191,23 @@ class CudaElementwiseFunction(ImplementationFor):
         return t0
 
 
+class CudaFunctionAndDerivative(ImplementationFor):
+    """What two calls of CudaElementwiseFunction with DerivIdx -1 and 0 compute, in one pass: drain, derivative's drain, source."""
+
+    def __init__(self, fun: int):
+        self.fun = fun
+
+    def run(self, call: ExecutionCall) -> Tensor:
+        dev = call.device
+        t0, t1, t2 = call.input(0), call.input(1), call.input(2)
+        dt = _same_type(call, 3)
+        k0, c0 = _cfg(t0); k1, c1 = _cfg(t1); k2, c2 = _cfg(t2)
+        L.check(L.lib.nk_unary_both(dev.ctx, self.fun, dt, t0.rank, t0._data.buf, c0, t1._data.buf, c1, t2._data.buf, c2), dev.ctx)
+        t0.version += 1
+        t1.version += 1
+        return t0
+
+
 class CudaScalarFunction(ImplementationFor):
     """ScalarAlgorithm (algorithms/ScalarAlgorithm.java:17-53; CLScalarFunction.java:19-27): a one-element
     tensor in, a one-element tensor out. Evaluated by the device's own scalar code, not on the host."""

@@ -358,14 +358,14 @@ def run_function(fid: str, x: Tensor, d: int = -1) -> Tensor:
 
 def run_function_and_derivative(fid: str, x: Tensor) -> Tuple[Tensor, Tensor]:
     """run_function(fid, x) and run_function(fid, x, 0), the eager local derivative of the backward pass, in one pass over x."""
-    if fid not in L.FUN or x.is_virtual or x.size == 1 or x.device is None:
+    if fid not in L.FUN or x.is_virtual or x.size == 1:
         return run_function(fid, x), run_function(fid, x, 0)
-    dev = x.device
+    dev = _common_device([x])
+    impl = B.backend().implementation_for(fid, B.ELEMENTWISE)
+    if type(impl) is not B.CudaElementwiseFunction:   # registered in its place: it answers for both
+        return run_function(fid, x), run_function(fid, x, 0)
     out, deriv = _new_output(x.dtype, x.shape, dev), _new_output(x.dtype, x.shape, dev)
-    (k0, c0), (kd, cd), (k1, c1) = B._cfg(out), B._cfg(deriv), B._cfg(x)
-    L.check(L.lib.nk_unary_both(dev.ctx, L.FUN[fid], B.nk_dtype(x.dtype), x.rank, out._data.buf, c0, deriv._data.buf, cd, x._data.buf, c1), dev.ctx)
-    out.version += 1
-    deriv.version += 1
+    _execute_on_common_device(ExecutionCall([out, deriv, x], fid, dev, -1), B.CudaFunctionAndDerivative(impl.fun))
     return out, deriv
 
 

@@ -350,3 +350,35 @@ def test_an_error_that_is_a_view_reaches_a_lower_rank_operand(device, op):
         f(a, b).backward(e)
         assert a.gradient.shape == (n,) and np.array_equal(a.gradient.items, want)
         assert np.array_equal(b.gradient.items, want if op == "+" else -want)
+
+
+def test_a_registered_implementation_of_a_function_is_used_with_and_without_gradients(device):
+    """The table decides what executes a function: an implementation put in the place of the built-in one also serves the eager
+    derivative of the backward pass."""
+    from neureka_b200 import backend as Bk
+
+    class Counting(Bk.CudaElementwiseFunction):
+        derivatives = []
+
+        def run(self, call):
+            self.derivatives.append(call.deriv_idx)
+            return super().run(call)
+
+    table, key = Bk.backend()._table, ("tanh", Bk.ELEMENTWISE)
+    built_in = table[key]
+    x_h = np.linspace(-2, 2, 24).astype(np.float32)
+    f = Function.of("tanh(i0)")
+
+    def step():
+        x = Tensor.of(np.float32, [4, 6], x_h).set_rqs_gradient(True).to(device)
+        y = f(x)
+        y.backward()
+        return y.items, x.gradient.items
+    want = step()
+    Bk.backend()._set("tanh", Bk.ELEMENTWISE, Counting(built_in.fun))
+    try:
+        got = step()
+    finally:
+        table[key] = built_in
+    assert Counting.derivatives == [-1, 0]
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
