@@ -182,7 +182,8 @@ int nk_sum_static(nk_ctx* ctx, int32_t dtype, int32_t rank, nk_buf* src, const i
 /* ---- routing knobs / introspection (no reference counterpart; measurement support) ---- */
 int nk_set_conv_path(nk_ctx* ctx, int32_t path);        /* nk_conv_path */
 int nk_last_conv_path(nk_ctx* ctx, int32_t* out_path);   /* family the last nk_conv used */
-const char* nk_last_kernel(nk_ctx* ctx);                 /* name of the last kernel launched */
+const char* nk_last_kernel(nk_ctx* ctx);                 /* name of the last kernel launched; two names stand for a family: nk_conv_gemm_kernel
+                                                          * (F64: nk_conv_dgemm_kernel) and nk_fused_kernel (with nk_fused_flat32) */
 int nk_launch_count(nk_ctx* ctx, uint64_t* out);         /* kernels launched by this ctx so far */
 int nk_timer_begin(nk_ctx* ctx);                         /* CUDA event on the ctx stream */
 int nk_timer_end(nk_ctx* ctx, float* out_ms);            /* second event + synchronise */

@@ -499,7 +499,7 @@ int tc_launch(nk_ctx* ctx, float* out, int64_t M, int64_t N, int64_t Kp, const f
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, kern, out, mAhi, mAlo, mBhi, mBlo, tp);
     if (e != cudaSuccess) return nk_cuda_fail(ctx, e, "cudaLaunchKernelEx(nk_conv_tc_kernel)");
-    return nk_after_launch(ctx, "nk_conv_tc_kernel<3xtf32>");
+    return nk_after_launch(ctx, CG == 2 ? "nk_conv_tc_kernel<3xtf32,pair>" : "nk_conv_tc_kernel<3xtf32>");
 }
 
 }  // namespace

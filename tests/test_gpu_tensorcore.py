@@ -49,7 +49,7 @@ def test_large_products_are_routed_to_the_tensor_cores_by_themselves(device, ora
     assert device.last_conv_path() == L.NK_CONV_GEMM
     mag = np.abs(a.reshape(m, k)).astype(np.float64) @ np.abs(b.reshape(k, n)).astype(np.float64)
     assert np.all(np.abs(auto.astype(np.float64) - fma) <= 1e-5 * mag.reshape(-1))
-    # F64 has no tensor-core route: the FMA family keeps it
+    # F64 has no tcgen05 route: the contraction family keeps it, on FP64 matrix instructions
     gpu_conv(device, np.zeros(m * n), c0, a.astype(np.float64), c1, b.astype(np.float64), c2)
     assert device.last_conv_path() == L.NK_CONV_GEMM
 
@@ -158,3 +158,37 @@ def test_products_split_along_k(device, mkn, order):
     runs = [gpu_conv(device, np.zeros(m * n, dtype=F32), ND.of_shape([m, 1, n]), a, ca, b, cb, path=L.NK_CONV_TC) for _ in range(2)]
     assert np.array_equal(runs[0], runs[1])
     assert np.all(np.abs(runs[0].reshape(m, n) - A @ B) <= 1e-5 * (np.abs(A) @ np.abs(B)))
+
+
+@pytest.mark.parametrize("mkn,pair", [((1999, 70, 2048), True), ((2048, 33, 1921), True), ((2300, 136, 2300), True), ((512, 256, 512), False),
+                                      ((64, 512, 64), False), ((130, 4001, 129), False), ((64, 9000, 500), False)])
+def test_which_shape_of_the_kernel_runs(device, mkn, pair):
+    """Pairs of CTAs where their tiles fill the chip, lone CTAs (k split where even these are few) otherwise."""
+    m, k, n = mkn
+    a, b = (np.ones(s, dtype=F32) for s in (m * k, k * n))
+    got = gpu_conv(device, np.zeros(m * n, dtype=F32), ND.of_shape([m, 1, n]), a, ND.of_shape([m, k, 1]), b, ND.of_shape([1, k, n]), path=L.NK_CONV_TC)
+    assert device.last_kernel() == ("nk_conv_tc_kernel<3xtf32,pair>" if pair else "nk_conv_tc_kernel<3xtf32>")
+    assert np.all(got == k)
+
+
+@pytest.mark.parametrize("k2", [70, 67])
+def test_products_split_along_k_through_offset_tables(device, k2):
+    """Several dims per index group and a drain in another order of its dims: the groups go through offset tables while k is split over
+    several CTAs. The sums are the ones of the same product written as plain matrices, which needs no tables: bit for bit."""
+    m1, m2, k1, n = 8, 17, 60, 97
+    m, k = m1 * m2, k1 * k2
+    rng = np.random.default_rng(k2)
+    a, b = rng.standard_normal(m * k).astype(F32), rng.standard_normal(k * n).astype(F32)
+    plain = gpu_conv(device, np.zeros(m * n, dtype=F32), ND.of_shape([m, 1, n]), a, ND.of_shape([m, k, 1]), b, ND.of_shape([1, k, n]), path=L.NK_CONV_TC)
+    A, B = a.reshape(m, k).astype(np.float64), b.reshape(k, n).astype(np.float64)
+    assert np.all(np.abs(plain.reshape(m, n) - A @ B) <= 1e-5 * (np.abs(A) @ np.abs(B)))
+    ca, cb, c0 = ND.of_shape([m1, m2, k1, k2, 1]), ND.of_shape([1, 1, k1, k2, n]), ND.of_shape([m1, m2, 1, 1, n])
+    tables = gpu_conv(device, np.zeros(m * n, dtype=F32), c0, a, ca, b, cb, path=L.NK_CONV_TC)
+    assert device.last_conv_path() == L.NK_CONV_TC and np.array_equal(tables, plain)
+    # operands stored with their dims the other way round, drain [n][m2][m1] in memory
+    at = a.reshape(m1, m2, k1, k2).transpose(3, 2, 1, 0).copy().reshape(-1)
+    bt = b.reshape(k1, k2, n).transpose(2, 1, 0).copy().reshape(-1)
+    ca, cb = ND.of_shape([1, k2, k1, m2, m1]).reshaped([4, 3, 2, 1, 0]), ND.of_shape([n, k2, k1, 1, 1]).reshaped([4, 3, 2, 1, 0])
+    c0 = ND.of_shape([n, 1, 1, m2, m1]).reshaped([4, 3, 2, 1, 0])
+    turned = gpu_conv(device, np.zeros(m * n, dtype=F32), c0, at, ca, bt, cb, path=L.NK_CONV_TC)
+    assert np.array_equal(turned.reshape(n, m2, m1).transpose(2, 1, 0).reshape(-1), plain)
