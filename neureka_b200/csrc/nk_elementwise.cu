@@ -67,9 +67,7 @@ __global__ void __launch_bounds__(256) nk_broadcast_reduce_kernel(T* __restrict_
             o0 += idx * p.s0[k]; o1 += idx * p.p1[k]; o2 += idx * p.p2[k];
         }
         T value = 0;
-        if (p.nred == 0) {
-            value += nkf::bin<0>(op, d, t1[o1], t2[o2]);
-        } else if (p.nred == 1) {
+        if (p.nred == 1) {   // (at least one dim is reduced: nothing reduced is an elementwise call)
             for (int64_t r = 0; r < p.rext[0]; r++) value += nkf::bin<0>(op, d, t1[o1 + r * p.r1[0]], t2[o2 + r * p.r2[0]]);
         } else {
             int64_t q[NK_MAX_RANK];
