@@ -126,8 +126,8 @@ __device__ __forceinline__ float sig32(float x) {
     const float y = float(sig_lean(double(fminf(fmaxf(x, -700.0f), 700.0f))));
     return x != x ? x + x : y;
 }
-// gelu's sigmoid as its derivative uses it, rounded to F32 by itself. This and sig32 give the bits of float(sig64(..)) for all
-// 2^32 inputs (swept), so the derivatives below lost nothing with the library's exp and division.
+// gelu's sigmoid as its derivative uses it, rounded to F32 by itself. The derivatives of sig, silu and gelu, which start from this and
+// sig32, were checked against the oracle on every 16th bit pattern.
 __device__ __forceinline__ float gelu_sig32(float x) {
     const float y = float(sig_lean(double(fminf(fmaxf(x, -411.0f), 411.0f)) * 1.702));
     return x != x ? x + x : y;

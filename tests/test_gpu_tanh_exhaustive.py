@@ -69,6 +69,35 @@ def test_silu_and_gelu_f32_on_every_16th_bit_pattern(device, oracle, fun):
     assert _sweep(device, oracle, fun, -1, 16) <= 1 << 14
 
 
+@pytest.mark.parametrize("fun,bound", [("sig", 2.0 ** -23), ("silu", 19 * 2.0 ** -24 + 2.0 ** -23), ("gelu", 19 * 2.0 ** -24 + 2.0 ** -23)])
+def test_derivatives_on_the_lean_sigmoid_f32_on_every_16th_bit_pattern(device, oracle, fun, bound):
+    """s (1 - s), s + x s (1 - s) and the same with 1.702 x (ScalarSigmoid.java, ScalarSiLU.java, ScalarGeLU.java), s rounded to F32 first.
+    Where two exp routines leave s one unit (2^-24 at most) apart the result moves by that times |1 - 2s| or |1 + x (1 - 2s)|, and |x| (or
+    1.702 |x|) is below 18 where s is neither 0 nor 1 to the last bit; 2^-23 more for the roundings. Few inputs differ at all."""
+    n, step, differing = 1 << 26, 16, 0
+    cfg = ND.of_shape([n])
+    inline = cfg.as_inline_array()
+    want = np.empty(n, dtype=np.float32)
+    for i in range((1 << 32) // (n * step)):
+        x = ((np.arange(i * n, (i + 1) * n, dtype=np.uint64) * step) + 5).astype(np.uint32).view(np.float32)
+        got = gpu_unary(device, L.FUN[fun], np.empty(n, dtype=np.float32), cfg, x, cfg, d=0)
+        oracle.unary(fun, want, inline, x, inline, d=0, threads=16)
+        idx = np.flatnonzero(got.view(np.int32) != want.view(np.int32))
+        g, w = got[idx], want[idx]
+        nan = np.isnan(w)
+        assert np.array_equal(np.isnan(g), nan)
+        g, w = g[~nan].astype(np.float64), w[~nan].astype(np.float64)
+        assert np.all(np.abs(g - w) <= bound), (fun, np.abs(g - w).max())
+        differing += g.size
+    assert differing <= 1 << 14
+    # infinities and NaN, which the clamps inside the sigmoid must not swallow
+    edge = np.array([np.inf, -np.inf, np.nan, 3e38, -3e38, 0.0, -0.0, 411.5, -411.5, 701.0, -701.0], dtype=np.float32)
+    c = ND.of_shape([edge.size])
+    want = np.empty(edge.size, dtype=np.float32)
+    oracle.unary(fun, want, c.as_inline_array(), edge, c.as_inline_array(), d=0)
+    assert np.array_equal(gpu_unary(device, L.FUN[fun], np.zeros(edge.size, dtype=np.float32), c, edge, c, d=0), want, equal_nan=True)
+
+
 def test_tanh_derivative_f32_on_a_dense_sample_of_bit_patterns(device, oracle):
     """tanh' = 1 - tanh(x)^2 with the float-rounded inner tanh (ScalarTanh.java:33-34): every 64th bit pattern."""
     n = 1 << 26
