@@ -68,8 +68,7 @@ def _broadcast_reduce(sym_op: int, target_like: Tensor, handle: Tensor, error: T
 
 def _zeros_view(dev, dtype, shape) -> Tensor:
     """A tensor of zeros of this shape that is one element of device memory (every index maps to it): the handle of the
-    backward-broadcast kernel of a sum or difference, of which only the shape matters. The kernel reads the element once; a
-    zero-filled array of the other operand's size took 120 of the 122 ms of a training step over 2^26 elements to build and move."""
+    backward-broadcast kernel of a sum or difference, of which only the shape matters. The kernel reads the element once."""
     from .ndconf import NDConfiguration
     t = Tensor(dtype, NDConfiguration.virtual_of(shape), None)
     t._attach(dev.allocate_from_one(dtype, 1, 0), dev)

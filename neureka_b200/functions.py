@@ -211,8 +211,8 @@ def _execute_on_common_device(call: ExecutionCall, impl) -> Tensor:
 
 def _new_output(dtype, shape, device: CudaDevice) -> Tensor:
     """The drain of a call. The reference hands the implementation a zero-filled tensor; every kernel of the path writes
-    every element of its drain, so the block is only allocated here. Building the zeros on the host and copying them up took
-    longer than the kernels that overwrote them: 0.51 s of a 2 ms training step over 2^26 elements."""
+    every element of its drain, so the block is only allocated here (2^26 zeros from the host take 120 ms, the kernel that overwrites
+    them 0.1)."""
     out = device.new_tensor(dtype, shape)
     out.is_intermediate = True
     return out
