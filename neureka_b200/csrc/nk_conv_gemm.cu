@@ -201,7 +201,8 @@ __device__ __forceinline__ void dg_mma(double (&c)[2], double a, double b) {
 }
 // TABLES: some index group goes through an offset table. Otherwise an element's address is one base per operand and thread plus
 // a constant step, moved on by a panel at a time: with the offsets worked out per element, the integer chains took longer than
-// the products (777 x 1023 x 515: 59 us, with offsets per element 79; 128 x 64 tiles of multiply-adds: 172).
+// the products (777 x 1023 x 515: 60 us, with offsets per element 79; 128 x 64 tiles of multiply-adds: 172). Through tables, 1024^3 in
+// groups of 32 x 32: 121 us, both offsets looked up per element 168.
 template <bool TABLES>
 __global__ void __launch_bounds__(128, 3) nk_conv_dgemm_kernel(double* __restrict__ out, const double* __restrict__ A, const double* __restrict__ B,
                                                                const GemmView p, const DgemmSplit sp) {
@@ -247,20 +248,36 @@ __global__ void __launch_bounds__(128, 3) nk_conv_dgemm_kernel(double* __restric
         }
         w.at += w.panel;
     };
+    // through tables: the rows' offsets are looked up once per tile, a panel's k offsets once per thread (k fastest) or element
+    __shared__ int64_t row_a[TABLES ? DG_T : 1], row_b[TABLES ? DG_T : 1];
+    if constexpr (TABLES) {
+        if (tid < DG_T) row_a[tid] = m0 + tid < p.M ? p.bA + p.Am.at(m0 + tid) : 0;
+        else row_b[tid - DG_T] = n0 + tid - DG_T < p.N ? p.bB + p.Bn.at(n0 + tid - DG_T) : 0;
+        __syncthreads();
+    }
+    auto gather = [&](const double* base, const int64_t* rows, const GemmOff& K, int64_t row0, int64_t n_rows, int kfast, int64_t k0, double (&v)[8]) {
+        int r, k;
+        place(kfast, 0, &r, &k);
+        if (kfast) {
+            const bool ok = k0 + k < k_end;
+            const int64_t ko = ok ? K.at(k0 + k) : 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = ok && row0 + r + 8 * i < n_rows ? base[rows[r + 8 * i] + ko] : 0.0;
+        } else {
+            const bool ok = row0 + r < n_rows;
+            const int64_t ro = rows[r];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = ok && k0 + k + 2 * i < k_end ? base[ro + K.at(k0 + k + 2 * i)] : 0.0;
+        }
+    };
     auto fetch = [&](int64_t k0) {
         if constexpr (!TABLES) {
             const int left = k_end - k0 < DG_K ? int(k_end - k0) : DG_K;
             pull(wa, sp.a_kfast, left, ra);
             pull(wb, sp.b_kfast, left, rb);
         } else {
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                int r, k;
-                place(sp.a_kfast, i, &r, &k);
-                ra[i] = m0 + r < p.M && k0 + k < k_end ? A[p.bA + p.Am.at(m0 + r) + p.Ak.at(k0 + k)] : 0.0;
-                place(sp.b_kfast, i, &r, &k);
-                rb[i] = n0 + r < p.N && k0 + k < k_end ? B[p.bB + p.Bn.at(n0 + r) + p.Bk.at(k0 + k)] : 0.0;
-            }
+            gather(A, row_a, p.Ak, m0, p.M, sp.a_kfast, k0, ra);
+            gather(B, row_b, p.Bk, n0, p.N, sp.b_kfast, k0, rb);
         }
     };
     auto stash = [&](int buf) {

@@ -481,3 +481,25 @@ def test_the_padded_copy_of_few_long_rows_uses_the_whole_chip(device):
             best = min(best, ms.value)
         return best
     assert best_ms(1_000_003) < 8 * best_ms(1_000_004)
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("dims", [((10, 10), (10, 10), 300), ((8, 17), (60, 67), 97), ((5, 13), (9, 31), 515)])
+def test_contractions_through_offset_tables_give_the_bits_of_plain_matrices(device, dt, dims):
+    """Several dims per index group, operands with k and with their rows contiguous, whole and partial tiles and panels, one and several
+    parts along k: the sums run in the same order as those of the same product of plain matrices, which needs no tables."""
+    (m1, m2), (k1, k2), n = dims
+    m, k = m1 * m2, k1 * k2
+    rng = np.random.default_rng(m + k)
+    a, b = rng.standard_normal(m * k).astype(dt), rng.standard_normal(k * n).astype(dt)
+    plain = gpu_conv(device, np.zeros(m * n, dtype=dt), ND.of_shape([m, 1, n]), a, ND.of_shape([m, k, 1]), b, ND.of_shape([1, k, n]), path=L.NK_CONV_GEMM)
+    shapes = [m1, m2, 1, 1, n], [m1, m2, k1, k2, 1], [1, 1, k1, k2, n]
+    c0, ca, cb = (ND.of_shape(s) for s in shapes)
+    got = gpu_conv(device, np.zeros(m * n, dtype=dt), c0, a, ca, b, cb, path=L.NK_CONV_GEMM)
+    assert device.last_conv_path() == L.NK_CONV_GEMM and np.array_equal(got, plain)
+    # every tensor stored with its dims the other way round
+    turn = [4, 3, 2, 1, 0]
+    t0, ta, tb = (ND.of_shape(s[::-1]).reshaped(turn) for s in shapes)
+    at, bt = (x.reshape(s).transpose(turn).copy().reshape(-1) for x, s in ((a, shapes[1]), (b, shapes[2])))
+    got = gpu_conv(device, np.zeros(m * n, dtype=dt), t0, at, ta, bt, tb, path=L.NK_CONV_GEMM)
+    assert np.array_equal(got.reshape(shapes[0][::-1]).transpose(turn).reshape(-1), plain)
