@@ -77,8 +77,10 @@ def _zeros_view(dev, dtype, shape) -> Tensor:
 
 
 def _is_whole(t: Tensor) -> bool:
-    """A tensor of its own in row-major order, which can be handed on or viewed in another shape: not a view, not one virtual element."""
-    return not t.is_virtual and not t.is_slice() and t.ndconf.is_simple()
+    """A tensor of its own in row-major order, which can be handed on or viewed in another shape: not a view, not one virtual element, not
+    column-major (whose elements another shape would name in another order)."""
+    c = t.ndconf
+    return not t.is_virtual and not t.is_slice() and c.strides == c.indices_map and c.is_compact()
 
 
 def _record_operator(sym: str, a: Tensor, b: Tensor, out: Tensor) -> None:

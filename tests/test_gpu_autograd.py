@@ -382,3 +382,17 @@ def test_a_registered_implementation_of_a_function_is_used_with_and_without_grad
         table[key] = built_in
     assert Counting.derivatives == [-1, 0]
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("op", ["+", "-"])
+def test_a_column_major_error_reaches_a_lower_rank_operand(device, op):
+    """The error of a sum that sums nothing, stored column-major: the gradient of an operand of lower rank has the error's elements in
+    the error's index order, not in the order of its memory."""
+    from neureka_b200.ndconf import Layout
+    e_h = np.arange(12, dtype=np.float32) + 1
+    e = Tensor.of(np.float32, [1, 3, 4], e_h).to_layout(Layout.COLUMN_MAJOR).to(device)
+    assert e.ndconf.layout() is Layout.COLUMN_MAJOR and np.array_equal(e.items, e_h)
+    a, b = (Tensor.of(np.float32, s, np.zeros(12)).set_rqs_gradient(True).to(device) for s in ([3, 4], [1, 3, 4]))
+    Function.of(f"i0 {op} i1")(a, b).backward(e)
+    assert np.array_equal(a.gradient.items, e_h)
+    assert np.array_equal(b.gradient.items, e_h if op == "+" else -e_h)
